@@ -409,8 +409,8 @@ mms_status mms_autotune(mms_ctx *ctx, int reps, int *cells_per_thread, int *zchu
 /* No counterpart in the reference.  n independent domains (each its own
  * deck: sizes, cooling, nucleation) stepped together on one device: per
  * step one CUDA graph with every domain's nucleation, activation, list and
- * capture as parallel branches and one persistent stencil launch over the
- * tiles of all domains.  All params[i] must share precision and device.
+ * capture as parallel branches and one stencil launch over the tiles of all
+ * domains.  All params[i] must share precision and device.
  * Each domain's state is exactly what mms_step would give it alone. */
 typedef struct mms_batch mms_batch;
 mms_status mms_batch_create(int n, const mms_params *params, mms_batch **out);
@@ -420,10 +420,10 @@ int mms_batch_size(const mms_batch *b);
  * records (not for mms_step while it belongs to the batch). */
 mms_ctx *mms_batch_domain(mms_batch *b, int i);
 mms_status mms_batch_step(mms_batch *b, int nsteps);
-/* Stencil tile of the persistent launch (as mms_set_stencil_tile). */
+/* Stencil tile of that launch (as mms_set_stencil_tile). */
 mms_status mms_batch_set_stencil_tile(mms_batch *b, int cells_per_thread, int zchunk);
 mms_status mms_batch_get_stencil_tile(const mms_batch *b, int *cells_per_thread, int *zchunk, int *grid);
-/* Times the persistent stencil for every tile candidate on shadows of the
+/* Times the batched stencil for every tile candidate on shadows of the
  * fields it writes and keeps the fastest. */
 mms_status mms_batch_autotune(mms_batch *b, int reps, int *cells_per_thread, int *zchunk, double *best_ms);
 uint64_t mms_batch_kernel_launches(const mms_batch *b);

@@ -137,6 +137,7 @@ struct mms_ctx {
     double *d_hred = nullptr;
     uint64_t launches = 0;
     bool stepped = false;
+    bool batched = false;  // stepped by an mms_batch
     std::string err;
     size_t bytes = 0;
     std::vector<void *> allocs;
@@ -263,6 +264,30 @@ void drop_graph(mms_ctx *ctx)
     ctx->multi_graph = nullptr;
     if (ctx->sum_graph) cudaGraphExecDestroy(ctx->sum_graph);
     ctx->sum_graph = nullptr;
+}
+
+// Every tile counts as changed: after any write of fields from outside a
+// step, and when the tiles themselves change (ordered on the stream).
+cudaError_t touch_tiles(mms_ctx *ctx)
+{
+    const TileMap &tm = ctx->ka.d.tm;
+    if (!tm.chg) return cudaSuccess;
+    long long tiles, edges;
+    tile_map_max(ctx->ka.g, &tiles, &edges);
+    return cudaMemsetAsync(tm.chg, 1, (size_t)tiles, ctx->stream);
+}
+
+// The tensor maps and the tile map for the context's tile choice.
+cudaError_t set_tiles(mms_ctx *ctx)
+{
+    make_tma(ctx->ka, ctx->prec, ctx->tma);
+    TileMap &tm = ctx->ka.d.tm;
+    tile_geometry(ctx->ka, ctx->tma);
+    // a domain whose tiles all run at once gains nothing from leaving some out
+    // (64^3: 32 us a step without the map, 35 with); in a batch they share the
+    // device with other domains' tiles
+    tm.on = tm.chg && ctx->tma.ok && (ctx->batched || tm.n > 148 * 4);
+    return touch_tiles(ctx);
 }
 
 void dfree(mms_ctx *ctx, void *p)
@@ -766,7 +791,7 @@ mms_status mms_set_stencil_tile(mms_ctx *ctx, int cells_per_thread, int zchunk)
     CU(cudaStreamSynchronize(ctx->stream));
     ctx->tma.cpt = cells_per_thread;
     ctx->tma.zc = zchunk;
-    make_tma(ctx->ka, ctx->prec, ctx->tma);
+    CU(set_tiles(ctx));
     drop_graph(ctx);
     ctx->fs_part_valid = false;
     if (ctx->nslabs == 1) prepare_graphs(ctx);
@@ -816,6 +841,7 @@ mms_status mms_autotune(mms_ctx *ctx, int reps, int *cells_per_thread, int *zchu
     const size_t N = (size_t)g.N;
     const size_t rs = ctx->prec == MMS_PREC_F32 ? sizeof(float) : sizeof(double);
     KernelArgs sa = ctx->ka;
+    sa.d.tm.on = 0;  // every tile, and no record of them
     const int pout = (int)((ctx->h_ctl->timestep + 1) & 1ULL);
     std::vector<void *> shadow;
     // es > 0: a field, placed as dalloc_field places it (es = its element size)
@@ -959,7 +985,7 @@ mms_status mms_autotune(mms_ctx *ctx, int reps, int *cells_per_thread, int *zchu
     ctx->tma.cpt = pick.cpt;
     ctx->tma.zc = pick.zc;
     ctx->am_rows = am_rows;
-    make_tma(ctx->ka, ctx->prec, ctx->tma);
+    CU(set_tiles(ctx));
     drop_graph(ctx);
     if (ctx->nslabs == 1) prepare_graphs(ctx);
     if (cells_per_thread) *cells_per_thread = pick.cpt;
@@ -1341,7 +1367,16 @@ mms_status create_ctx(const mms_params *pin, int nslabs, int slab, mms_ctx **out
             (st = alloc_slab_rows(ctx, slab_capacity(ctx, thr))))
             return fail(st);
     }
-    make_tma(ctx->ka, ctx->prec, ctx->tma);
+    if (nslabs == 1) {
+        // the tile map (a slab visits every tile: its neighbours' planes change its halo)
+        TileMap &tm = d.tm;
+        long long tiles, edges;
+        tile_map_max(g, &tiles, &edges);
+        if ((st = dalloc(ctx, &tm.chg, (size_t)tiles)) || (st = dalloc(ctx, &tm.keep_x, (size_t)tiles)) ||
+            (st = dalloc(ctx, &tm.act, (size_t)tiles)) || (p.am && (st = dalloc(ctx, &tm.am_max, 4 + 400 * (size_t)edges))))
+            return fail(st);
+    }
+    if (set_tiles(ctx) != cudaSuccess) return fail(MMS_ERR_CUDA);
     // orientation tables
     if (p.gnUseOrientation) {
         long long maxsites = 0;
@@ -1819,6 +1854,7 @@ mms_status mms_upload(mms_ctx *ctx, mms_field field, const void *host)
     const size_t N = (size_t)g.N;
     mms_status st;
     DevPtrs &d = ctx->ka.d;
+    CU(touch_tiles(ctx));
     switch (field) {
     case MMS_FIELD_CE:
     case MMS_FIELD_CL:
@@ -2062,6 +2098,7 @@ void adj_stop_recording(mms_ctx *ctx)
         d.rec_flags = nullptr;
         d.rec_curv = nullptr;
         d.rec_cap = 0;
+        touch_tiles(ctx);  // the recording stencil keeps no tile map
         drop_graph(ctx);
     }
 }
@@ -2315,7 +2352,7 @@ mms_status mms_adjoint_gradient(mms_ctx *ctx, const double *target_ce, mms_adjoi
 // ============================================================ batched domains
 // Many independent domains stepped together: one CUDA graph per step holds
 // every domain's nucleation and activation (parallel branches), ONE
-// persistent stencil launch over the tiles of all domains, and every
+// stencil launch over the tiles of all domains, and every
 // domain's list and capture (parallel branches).
 struct mms_batch {
     std::vector<mms_ctx *> doms;
@@ -2326,6 +2363,7 @@ struct mms_batch {
     std::vector<cudaEvent_t> ev_fork, ev_join;
     void *items = nullptr;  // device array of batch items
     long long total_tiles = 0;
+    unsigned char *act = nullptr;  // the tiles to visit, of all domains
     // prefix sums of the small kernels' blocks per domain (nucleation,
     // activation, list, capture), n + 1 each, on the device
     int *begin = nullptr;
@@ -2349,16 +2387,22 @@ void batch_drop_graph(mms_batch *b)
 // Kernel arguments of every domain (sites and tables can be replaced
 // between calls) and the small kernels' block prefixes; the step graph is
 // dropped when a launch's block total changed.
+mms_status batch_build_items(mms_batch *b);
+
 mms_status batch_refresh(mms_batch *b)
 {
     const size_t nd = b->doms.size(), ib = batch_item_bytes();
     if (!b->items) return MMS_OK;
+    // a domain given a tile of its own returns to the batch's: the tile flags
+    // and the stencil launch are sized for that one
+    for (const mms_ctx *ctx : b->doms)
+        if (ctx->tma.cpt != b->cpt || ctx->tma.zc != b->zc) return batch_build_items(b);
     std::vector<unsigned char> host(ib * nd);
     std::vector<int> begin(4 * (nd + 1), 0);
     long long tiles = 0;
     for (size_t i = 0; i < nd; i++) {
         mms_ctx *ctx = b->doms[i];
-        tiles += fill_batch_item(host.data() + ib * i, ctx->ka, ctx->tma, tiles);
+        tiles += fill_batch_item(host.data() + ib * i, ctx->ka, ctx->tma, tiles, b->act);
         for (int w = 0; w < 4; w++) begin[w * (nd + 1) + i + 1] = begin[w * (nd + 1) + i] + batch_blocks(ctx->ka, w);
     }
     if (!b->begin && cudaMalloc(&b->begin, sizeof(int) * begin.size()) != cudaSuccess) {
@@ -2386,15 +2430,25 @@ mms_status batch_build_items(mms_batch *b)
         mms_ctx *ctx = b->doms[i];
         ctx->tma.cpt = b->cpt;
         ctx->tma.zc = b->zc;
-        if (!make_tma(ctx->ka, ctx->prec, ctx->tma)) {
+        if (set_tiles(ctx) != cudaSuccess || !ctx->tma.ok) {
             b->err = "TMA descriptors could not be encoded for a batched domain";
             return MMS_ERR_CUDA;
         }
         drop_graph(ctx);
-        tiles += fill_batch_item(host.data() + ib * i, ctx->ka, ctx->tma, tiles);
+        tiles += ctx->ka.d.tm.n;
     }
     if (b->items) cudaFree(b->items);
+    if (b->act) cudaFree(b->act);
     b->items = nullptr;
+    b->act = nullptr;
+    if (cudaMalloc(&b->act, (size_t)tiles) != cudaSuccess ||
+        cudaMemsetAsync(b->act, 0, (size_t)tiles, b->stream) != cudaSuccess) {
+        b->err = "cudaMalloc of the batch's tile flags failed";
+        return MMS_ERR_NOMEM;
+    }
+    tiles = 0;
+    for (size_t i = 0; i < b->doms.size(); i++)
+        tiles += fill_batch_item(host.data() + ib * i, b->doms[i]->ka, b->doms[i]->tma, tiles, b->act);
     if (cudaMalloc(&b->items, host.size()) != cudaSuccess) {
         b->err = "cudaMalloc of the batch items failed";
         return MMS_ERR_NOMEM;
@@ -2411,7 +2465,7 @@ mms_status batch_build_items(mms_batch *b)
 // One step of every domain, on b->stream (captured into the step graph):
 // AM temperatures as parallel branches, then one launch each of nucleation
 // and activation over all domains, curvature branches (TipCurvature decks),
-// the persistent stencil, and one launch each of list and capture.
+// the stencil, and one launch each of list and capture.
 int batch_launch_step(mms_batch *b)
 {
     int n = 0;
@@ -2441,7 +2495,7 @@ int batch_launch_step(mms_batch *b)
         if (!ctx->p.tip_curv) return 0;
         return s ? launch_curv(ctx->ka, ctx->prec, s) : 1;
     });
-    n += launch_stencil_batch(b->items, nd, b->total_tiles, b->prec, b->cpt, b->grid, b->stream);
+    n += launch_stencil_batch(b->items, nd, b->total_tiles, b->prec, b->cpt, b->act, b->stream);
     n += launch_small_batch(2, b->items, bg + 2 * (nd + 1), nd, b->totals[2], b->prec, b->stream);
     n += launch_small_batch(3, b->items, bg + 3 * (nd + 1), nd, b->totals[3], b->prec, b->stream);
     return n;
@@ -2502,6 +2556,7 @@ mms_status mms_batch_destroy(mms_batch *b)
     for (mms_ctx *ctx : b->doms) mms_destroy(ctx);
     if (b->items) cudaFree(b->items);
     if (b->begin) cudaFree(b->begin);
+    if (b->act) cudaFree(b->act);
     for (cudaStream_t s : b->side) cudaStreamDestroy(s);
     for (cudaEvent_t e : b->ev_fork) cudaEventDestroy(e);
     for (cudaEvent_t e : b->ev_join) cudaEventDestroy(e);
@@ -2538,7 +2593,10 @@ mms_status mms_batch_create(int n, const mms_params *params, mms_batch **out)
         cudaEventCreateWithFlags(&b->ev_join[i], cudaEventDisableTiming);
     }
     for (auto &e : b->ev_fork) cudaEventCreateWithFlags(&e, cudaEventDisableTiming);
-    for (mms_ctx *ctx : b->doms) mms_set_stream(ctx, b->stream);
+    for (mms_ctx *ctx : b->doms) {
+        mms_set_stream(ctx, b->stream);
+        ctx->batched = true;
+    }
     mms_status st = batch_build_items(b);
     if (st) {
         mms_batch_destroy(b);
@@ -2627,7 +2685,7 @@ mms_status mms_batch_get_stencil_tile(const mms_batch *b, int *cells_per_thread,
     return MMS_OK;
 }
 
-// Batch tile autotuner: the persistent stencil over all domains is timed for
+// Batch tile autotuner: the stencil over all domains is timed for
 // every candidate tile on shadows of the fields it writes (as mms_autotune
 // does for one domain); the fastest by median of `reps` launches is kept.
 mms_status mms_batch_autotune(mms_batch *b, int reps, int *cells_per_thread, int *zchunk, double *best_ms)
@@ -2652,6 +2710,7 @@ mms_status mms_batch_autotune(mms_batch *b, int reps, int *cells_per_thread, int
         const Geo &g = ctx->ka.g;
         const size_t N = (size_t)g.N, rs = ctx->prec == MMS_PREC_F32 ? sizeof(float) : sizeof(double);
         KernelArgs sa = ctx->ka;
+        sa.d.tm.on = 0;  // every tile, and no record of them
         const int pout = (int)((ctx->h_ctl->timestep + 1) & 1ULL);
         // es > 0: a field, placed as dalloc_field places it
         auto sh = [&](const void *src, size_t bytes, size_t es = 0) -> void * {
@@ -2703,16 +2762,16 @@ mms_status mms_batch_autotune(mms_batch *b, int reps, int *cells_per_thread, int
                 th.cpt = cpt;
                 th.zc = zc;
                 ok = make_tma(sargs[i], b->prec, th) != 0;
-                tiles += fill_batch_item(host.data() + ib * i, sargs[i], th, tiles);
+                tiles += fill_batch_item(host.data() + ib * i, sargs[i], th, tiles, nullptr);
             }
             if (!ok) continue;
             cudaMemcpyAsync(ditems, host.data(), host.size(), cudaMemcpyHostToDevice, b->stream);
             cudaStreamSynchronize(b->stream);
-            const int grid = batch_grid(b->prec, cpt);
+            batch_grid(b->prec, cpt);  // the kernel's shared memory
             std::vector<float> ms;
             for (int r = 0; r < reps + 2; r++) {
                 cudaEventRecord(e0, b->stream);
-                launch_stencil_batch(ditems, (int)nd, tiles, b->prec, cpt, grid, b->stream);
+                launch_stencil_batch(ditems, (int)nd, tiles, b->prec, cpt, nullptr, b->stream);
                 cudaEventRecord(e1, b->stream);
                 cudaEventSynchronize(e1);
                 float t = 0.f;
@@ -2873,6 +2932,7 @@ mms_status mms_checkpoint_load(mms_ctx *ctx, const char *path)
         ctx->err = why;
         return s;
     };
+    if (touch_tiles(ctx) != cudaSuccess) return fail(MMS_ERR_CUDA, "the tile map could not be reset");
     if (!fread_all(fp, &h, sizeof h) || std::memcmp(h.magic, "MMSCKPT", 8) != 0 || h.version != 4)
         return fail(MMS_ERR_IO, "not a checkpoint of this library");
     if (h.prec != ctx->prec || h.gx != g.gx || h.gy != g.gy || h.gz != g.gz || h.nranks != g.nranks ||

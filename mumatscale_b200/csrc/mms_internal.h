@@ -151,6 +151,20 @@ struct Fields {
     Real *fs[2];
 };
 
+// Which stencil tiles a step has to visit (kernels.cu, "active tiles").
+// Tiles are those of the stencil's launch: (1 << wsh) x 8 x zc cells, nx x ny
+// x nz of them, tile index (bz ny + by) nx + bx.
+struct TileMap {
+    int on;                // 0: every tile is visited in every step
+    int nx, ny, nz, n;
+    int wsh, zc;
+    unsigned char *chg;    // per tile: not at rest
+    double *keep_x;        // per tile at rest: least m (cl - Cinit) of its solid cells (+inf: none)
+    unsigned char *act;    // per tile: to be visited in this step
+    float *am_max;         // AM: liniT and Tfront (doubles), then per tile column, row and
+                           // layer the largest X, Y and Z of each node (AM_NT contiguous)
+};
+
 struct DevPtrs {
     void *ce;
     void *cl[2];
@@ -224,6 +238,7 @@ struct DevPtrs {
     double *rec_curv;
     unsigned long long rec_t0;
     long long rec_cap;
+    TileMap tm;
 };
 
 // fs_change_diffuse branches (growth.c:228-272), as recorded for the adjoint
@@ -265,9 +280,14 @@ struct Profiler {
 // it launched.
 // start_stage 0: whole step; 1: resume at grain activation (after a stall).
 // sumfs: the TMA stencil also leaves its per-tile fraction-solid sums in
-// a.d.fs_part (see stencil_parts).
+// a.d.fs_part (see stencil_parts).  A resumed step visits every tile.
 int launch_step(const KernelArgs &a, const TmaHolder &tma, int precision, void *stream, int start_stage,
                 Profiler *prof, bool sumfs = false);
+// The tile geometry of the current stencil tile, into a.d.tm (its buffers
+// and `on` are the caller's); tile_map_max: the most tiles, columns + rows +
+// layers of tiles any choice gives.
+void tile_geometry(KernelArgs &a, const TmaHolder &tma);
+void tile_map_max(const Geo &g, long long *tiles, long long *edges);
 // Builds the TMA descriptors of the stencil for the current buffers;
 // returns 0 when the driver cannot encode them (the stencil then uses its
 // plain-load variant).
@@ -285,13 +305,16 @@ int launch_curv(const KernelArgs &a, int precision, void *stream);
 int launch_slab_phase(const KernelArgs &a, const TmaHolder &tma, int precision, void *stream, int phase,
                       int resume);
 // Batched stencil over many domains: one item per domain (opaque, built by
-// fill_batch_item, which returns the domain's tile count), one persistent
-// launch of batch_grid CTAs.
+// fill_batch_item, which returns the domain's tile count), one launch;
+// batch_grid: its CTAs resident at once.
 size_t batch_item_bytes();
-long long fill_batch_item(void *dst, const KernelArgs &a, const TmaHolder &tma, long long tile_begin);
+// (act: the batch's active-tile bytes, null: every tile)
+long long fill_batch_item(void *dst, const KernelArgs &a, const TmaHolder &tma, long long tile_begin,
+                          unsigned char *act);
 int batch_grid(int precision, int cpt);
-int launch_stencil_batch(const void *items, int nitems, long long total_tiles, int precision, int cpt, int grid,
-                         void *stream);
+// act: the tiles to visit, a byte each over all domains (null: every tile)
+int launch_stencil_batch(const void *items, int nitems, long long total_tiles, int precision, int cpt,
+                         const unsigned char *act, void *stream);
 // The other kernels of a step over all domains, one launch each: which = 0
 // nucleation, 1 activation, 2 interface list, 3 capture; begin: device
 // prefix sums (n + 1) of batch_blocks over the domains, total = begin[n].
