@@ -541,7 +541,9 @@ typedef struct mms_adjoint_result {
 mms_status mms_adjoint_record(mms_ctx *ctx, int nsteps, int checkpoint_every);
 /* Loss and gradient for the recorded run; target_ce in the halo'd layout
  * (FP64).  Each segment between checkpoints is recomputed from its
- * checkpoint by frozen replay, then differentiated backwards. */
+ * checkpoint by frozen replay, then differentiated backwards.  The work
+ * buffers (checkpoint_every states, two sets of adjoints) are made by the
+ * first call and kept until the record is released or replaced. */
 mms_status mms_adjoint_gradient(mms_ctx *ctx, const double *target_ce, mms_adjoint_result *out);
 /* Loss of the frozen replay of the whole recorded run from its first
  * checkpoint with Dliq, part_coef and GibbsThomsonCoef multiplied by

@@ -184,6 +184,14 @@ struct mms_ctx {
         unsigned char *flags = nullptr;  // nrec x N
         double *curv = nullptr;          // nrec x N (TipCurvature)
         char *ckpt = nullptr;            // nckpt x 3 x N x element size
+        // work buffers of the gradient and the replayed loss, made by the
+        // first of them and kept as long as the record
+        char *seg = nullptr;             // seg_states x 3 x N: replayed states, halos as recorded
+        long long seg_states = 0;        // 2 for the loss, at least `every` for the gradient
+        char *lam = nullptr;             // 6 x N: adjoints of (ce, cl, fs), two sets
+        double *tgt = nullptr;           // N
+        double *partial = nullptr;       // adj_nblocks x ADJ_SLOTS
+        double *acc = nullptr;           // ADJ_SLOTS gradient sums, then the loss
     } adj;
 };
 
@@ -2109,6 +2117,11 @@ void adj_free(mms_ctx *ctx)
     dfree(ctx, ctx->adj.flags);
     dfree(ctx, ctx->adj.curv);
     dfree(ctx, ctx->adj.ckpt);
+    dfree(ctx, ctx->adj.seg);
+    dfree(ctx, ctx->adj.lam);
+    dfree(ctx, ctx->adj.tgt);
+    dfree(ctx, ctx->adj.partial);
+    dfree(ctx, ctx->adj.acc);
     ctx->adj = mms_ctx::AdjRec{};
 }
 
@@ -2124,6 +2137,37 @@ mms_status adj_save_ckpt(mms_ctx *ctx, long long idx, unsigned long long ts)
         CU(cudaMemcpyAsync(state_slot(ctx->adj.ckpt, idx, f, N, es), src[f], N * es, cudaMemcpyDeviceToDevice,
                            ctx->stream));
     return MMS_OK;
+}
+
+// The work buffers of the record.  Allocated on the first call (128^3 FP64,
+// checkpoints every 50 steps: 2.6 GB, whose allocation, clearing and release
+// took about as long as the gradient itself when each call did them); the
+// replay writes interior cells, and no halo cell changes during a run, so the
+// states' halos are filled here once instead of copying the checkpoint into
+// every state.
+mms_status adj_buffers(mms_ctx *ctx, bool gradient)
+{
+    mms_ctx::AdjRec &r = ctx->adj;
+    const Geo &g = ctx->ka.g;
+    const size_t N = (size_t)g.N, es = elem_size(ctx);
+    const long long states = gradient ? std::max(2, r.every) : 2;
+    mms_status st = MMS_OK;
+    if (r.seg_states < states) {
+        CU(cudaStreamSynchronize(ctx->stream));
+        dfree(ctx, r.seg);
+        r.seg = nullptr;
+        r.seg_states = 0;
+        if ((st = dalloc(ctx, &r.seg, (size_t)states * 3 * N * es, false))) return st;
+        r.seg_states = states;
+        for (long long s = 0; s < states; s++)
+            CU(cudaMemcpyAsync(state_slot(r.seg, s, 0, N, es), state_slot(r.ckpt, 0, 0, N, es), 3 * N * es,
+                               cudaMemcpyDeviceToDevice, ctx->stream));
+    }
+    auto need = [&](auto **ptr, size_t n) { return *ptr ? MMS_OK : dalloc(ctx, ptr, n, false); };
+    if ((st = need(&r.tgt, N)) || (st = need(&r.partial, (size_t)adj_nblocks(g) * ADJ_SLOTS)) ||
+        (st = need(&r.acc, ADJ_SLOTS + 1)))
+        return st;
+    return gradient ? need(&r.lam, 6 * N * es) : MMS_OK;
 }
 
 // Phys with Dliq, part_coef and the Gibbs-Thomson coefficient scaled, each
@@ -2214,45 +2258,28 @@ mms_status mms_adjoint_replay_loss(mms_ctx *ctx, const double *target_ce, const 
     const size_t N = (size_t)g.N, es = elem_size(ctx);
     const mms_ctx::AdjRec &r = ctx->adj;
     const Phys ph = scaled_phys(ctx, scale);
-    char *buf = nullptr;
-    double *tgt = nullptr, *partial = nullptr, *dl = nullptr;
-    mms_status st;
-    auto cleanup = [&]() {
-        cudaStreamSynchronize(ctx->stream);
-        dfree(ctx, buf);
-        dfree(ctx, tgt);
-        dfree(ctx, partial);
-        dfree(ctx, dl);
-    };
-    if ((st = dalloc(ctx, &buf, 2 * 3 * N * es)) || (st = dalloc(ctx, &tgt, N)) ||
-        (st = dalloc(ctx, &partial, (size_t)adj_nblocks(g))) || (st = dalloc(ctx, &dl, 1))) {
-        cleanup();
-        return st;
-    }
-    cudaError_t e = copy_in(ctx, tgt, target_ce, sizeof(double));
-    for (int b = 0; b < 2 && e == cudaSuccess; b++)
-        for (int f = 0; f < 3 && e == cudaSuccess; f++)
-            e = cudaMemcpyAsync(state_slot(buf, b, f, N, es), state_slot(r.ckpt, 0, f, N, es), N * es,
-                                cudaMemcpyDeviceToDevice, ctx->stream);
-    int cur = 0;
+    mms_status st = adj_buffers(ctx, false);
+    if (st) return st;
+    cudaError_t e = copy_in(ctx, r.tgt, target_ce, sizeof(double));
+    // from the first checkpoint through two states in turn
+    const char *from = r.ckpt;
     for (long long s = 0; s < r.nrec && e == cudaSuccess; s++) {
-        const void *x0[3] = {state_slot(buf, cur, 0, N, es), state_slot(buf, cur, 1, N, es),
-                             state_slot(buf, cur, 2, N, es)};
-        void *x1[3] = {state_slot(buf, 1 - cur, 0, N, es), state_slot(buf, 1 - cur, 1, N, es),
-                       state_slot(buf, 1 - cur, 2, N, es)};
+        char *to = state_slot(r.seg, s & 1, 0, N, es);
+        const void *x0[3] = {from, from + N * es, from + 2 * N * es};
+        void *x1[3] = {to, to + N * es, to + 2 * N * es};
         launch_replay(g, ph, ctx->prec, x0, x1, r.flags + (size_t)s * N, r.curv ? r.curv + (size_t)s * N : nullptr,
                       r.t0 + s + 1, ctx->stream);
-        cur = 1 - cur;
+        from = to;
     }
     const double off = ctx->prec == MMS_PREC_F32 ? ctx->p.Cinit : 0.0;
     if (e == cudaSuccess) {
-        launch_adj_terminal(g, ctx->prec, off, state_slot(buf, cur, 0, N, es), tgt, nullptr, nullptr, nullptr,
-                            partial, dl, ctx->stream);
+        launch_adj_terminal(g, ctx->prec, off, from, r.tgt, nullptr, nullptr, nullptr, r.partial, r.acc + ADJ_SLOTS,
+                            ctx->stream);
         e = cudaGetLastError();
     }
-    if (e == cudaSuccess) e = cudaMemcpyAsync(loss, dl, sizeof(double), cudaMemcpyDeviceToHost, ctx->stream);
+    if (e == cudaSuccess)
+        e = cudaMemcpyAsync(loss, r.acc + ADJ_SLOTS, sizeof(double), cudaMemcpyDeviceToHost, ctx->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
-    cleanup();
     if (e != cudaSuccess) {
         ctx->err = std::string("adjoint replay: ") + cudaGetErrorString(e);
         return MMS_ERR_CUDA;
@@ -2271,65 +2298,49 @@ mms_status mms_adjoint_gradient(mms_ctx *ctx, const double *target_ce, mms_adjoi
     const size_t N = (size_t)g.N, es = elem_size(ctx);
     const mms_ctx::AdjRec &r = ctx->adj;
     const Phys &ph = ctx->ka.p;
-    const int nb = adj_nblocks(g);
-    char *seg = nullptr, *lam = nullptr;
-    double *tgt = nullptr, *partial = nullptr, *acc = nullptr;
-    mms_status st;
-    auto cleanup = [&]() {
-        cudaStreamSynchronize(ctx->stream);
-        dfree(ctx, seg);
-        dfree(ctx, lam);
-        dfree(ctx, tgt);
-        dfree(ctx, partial);
-        dfree(ctx, acc);
-    };
-    // acc: ADJ_SLOTS gradient sums, then the loss
-    if ((st = dalloc(ctx, &seg, (size_t)(r.every + 1) * 3 * N * es)) || (st = dalloc(ctx, &lam, 6 * N * es)) ||
-        (st = dalloc(ctx, &tgt, N)) || (st = dalloc(ctx, &partial, (size_t)nb * ADJ_SLOTS)) ||
-        (st = dalloc(ctx, &acc, ADJ_SLOTS + 1))) {
-        cleanup();
-        return st;
-    }
-    // adjoint buffers: lce, lcl[2], lfs[2], nu
-    char *lce = lam, *lcl[2] = {lam + N * es, lam + 2 * N * es}, *lfs[2] = {lam + 3 * N * es, lam + 4 * N * es},
-         *nu = lam + 5 * N * es;
-    cudaError_t e = copy_in(ctx, tgt, target_ce, sizeof(double));
+    mms_status st = adj_buffers(ctx, true);
+    if (st) return st;
+    cudaError_t e = copy_in(ctx, r.tgt, target_ce, sizeof(double));
     const double off = ctx->prec == MMS_PREC_F32 ? ctx->p.Cinit : 0.0;
+    auto adjoints = [&](int set, int f) { return r.lam + (size_t)(3 * set + f) * N * es; };
+    // state l of a segment: its checkpoint, then the replayed ones
+    auto state = [&](long long sg, long long l) {
+        return l == 0 ? state_slot(r.ckpt, sg, 0, N, es) : state_slot(r.seg, l - 1, 0, N, es);
+    };
     int lc = 0;
     for (long long sg = r.nckpt - 1; sg >= 0 && e == cudaSuccess; sg--) {
         const long long s0 = sg * r.every, s1 = std::min<long long>(s0 + r.every, r.nrec), L = s1 - s0;
-        // every slot starts as the checkpoint (halo cells never change)
-        for (long long l = 0; l <= L && e == cudaSuccess; l++)
-            for (int f = 0; f < 3 && e == cudaSuccess; f++)
-                e = cudaMemcpyAsync(state_slot(seg, l, f, N, es), state_slot(r.ckpt, sg, f, N, es), N * es,
-                                    cudaMemcpyDeviceToDevice, ctx->stream);
         for (long long l = 0; l < L; l++) {
-            const void *x0[3] = {state_slot(seg, l, 0, N, es), state_slot(seg, l, 1, N, es),
-                                 state_slot(seg, l, 2, N, es)};
-            void *x1[3] = {state_slot(seg, l + 1, 0, N, es), state_slot(seg, l + 1, 1, N, es),
-                           state_slot(seg, l + 1, 2, N, es)};
+            const char *from = state(sg, l);
+            char *to = state(sg, l + 1);
+            const void *x0[3] = {from, from + N * es, from + 2 * N * es};
+            void *x1[3] = {to, to + N * es, to + 2 * N * es};
             const size_t s = (size_t)(s0 + l);
             launch_replay(g, ph, ctx->prec, x0, x1, r.flags + s * N, r.curv ? r.curv + s * N : nullptr,
                           r.t0 + s + 1, ctx->stream);
         }
-        if (sg == r.nckpt - 1)
-            launch_adj_terminal(g, ctx->prec, off, state_slot(seg, L, 0, N, es), tgt, lce, lcl[lc], lfs[lc],
-                                partial, acc + ADJ_SLOTS, ctx->stream);
+        if (sg == r.nckpt - 1) {
+            // the loss; the blocks' sums of the gradient start at zero after it
+            launch_adj_terminal(g, ctx->prec, off, state(sg, L), r.tgt, adjoints(lc, 0), adjoints(lc, 1),
+                                adjoints(lc, 2), r.partial, r.acc + ADJ_SLOTS, ctx->stream);
+            e = cudaMemsetAsync(r.partial, 0, sizeof(double) * (size_t)adj_nblocks(g) * ADJ_SLOTS, ctx->stream);
+        }
         for (long long l = L - 1; l >= 0; l--) {
-            const void *x0[3] = {state_slot(seg, l, 0, N, es), state_slot(seg, l, 1, N, es),
-                                 state_slot(seg, l, 2, N, es)};
+            const char *from = state(sg, l);
+            const void *x0[3] = {from, from + N * es, from + 2 * N * es};
+            const void *l1[3] = {adjoints(lc, 0), adjoints(lc, 1), adjoints(lc, 2)};
+            void *l0[3] = {adjoints(1 - lc, 0), adjoints(1 - lc, 1), adjoints(1 - lc, 2)};
             const size_t s = (size_t)(s0 + l);
-            launch_adj_step(g, ph, ctx->prec, x0, state_slot(seg, l + 1, 0, N, es), r.flags + s * N,
-                            r.curv ? r.curv + s * N : nullptr, lce, lcl[lc], lfs[lc], lcl[1 - lc], lfs[1 - lc], nu,
-                            partial, acc, r.t0 + s + 1, ctx->stream);
+            launch_adj_step(g, ph, ctx->prec, x0, state(sg, l + 1), r.flags + s * N,
+                            r.curv ? r.curv + s * N : nullptr, l1, l0, r.partial, r.t0 + s + 1, ctx->stream);
             lc = 1 - lc;
         }
         if (e == cudaSuccess) e = cudaGetLastError();
     }
+    if (e == cudaSuccess) launch_adj_fold(g, r.partial, r.acc, ctx->stream);
     double h[ADJ_SLOTS + 1] = {};
-    if (e == cudaSuccess) e = cudaMemcpyAsync(h, acc, sizeof h, cudaMemcpyDeviceToHost, ctx->stream);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(h, r.acc, sizeof h, cudaMemcpyDeviceToHost, ctx->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
-    cleanup();
     if (e != cudaSuccess) {
         ctx->err = std::string("adjoint: ") + cudaGetErrorString(e);
         return MMS_ERR_CUDA;

@@ -372,10 +372,12 @@ constexpr int ADJ_SLOTS = 6;  // gradient slots: rl, D_xt, km, km_inv, k_inv, gi
 int adj_nblocks(const Geo &g);
 int launch_replay(const Geo &g, const Phys &p, int precision, const void *const x0[3], void *const x1[3],
                   const unsigned char *flags, const double *curv, unsigned long long ts, void *stream);
+// l1, l0: (lce, lcl, lfs), the adjoints after and before the step; partial:
+// adj_nblocks x ADJ_SLOTS running sums, which launch_adj_fold adds up
 int launch_adj_step(const Geo &g, const Phys &p, int precision, const void *const x0[3], const void *ce1,
-                    const unsigned char *flags, const double *curv, void *lce, const void *lcl1, const void *lfs1,
-                    void *lcl0, void *lfs0, void *nu, double *partial, double *grad, unsigned long long ts,
-                    void *stream);
+                    const unsigned char *flags, const double *curv, const void *const l1[3], void *const l0[3],
+                    double *partial, unsigned long long ts, void *stream);
+int launch_adj_fold(const Geo &g, const double *partial, double *grad, void *stream);
 int launch_adj_terminal(const Geo &g, int precision, double cinit_off, const void *ce, const double *target,
                         void *lce, void *lcl, void *lfs, double *partial, double *loss_out, void *stream);
 
