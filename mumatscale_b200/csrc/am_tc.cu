@@ -711,9 +711,34 @@ long long am_ximg_size(int gx, int gy, int gz)
     return am_ximg_part(gx) + (long long)(gy + gz + 4) * AM_NT + am_bimg_part(gy, gz);
 }
 
-// rows: 256-row tiles (one accumulator set), 64-128 rows (two), 0 = 256
-// when the grid has at least two 256-row tiles per SM, else 128.
-// With two sets a tile's epilogue overlaps the next tile's MMAs; 256-row
+// The rows per tile with the least expected time: rounds of tiles over the SMs
+// x rows x the measured time per row of each height (below), so that a small
+// grid does not leave most SMs idle in its last round (317 x 149 x 83: 128 rows
+// make 2.05 rounds, 96 rows 2.7; us per step with tables and image, 128 rows ->
+// so: 61.5 -> 59.5; 178 x 96 x 120 51.3 -> 48.2; 512 x 256 x 128 122 -> 97).
+int am_default_rows(const Geo &g)
+{
+    static const struct {
+        int rows;
+        double per_row;
+    } heights[] = {{256, 0.904}, {128, 1.0}, {112, 1.056}, {96, 1.112}, {80, 1.256}, {64, 1.424}};
+    const long long ntx = (g.gx + TC_M - 1) / TC_M, nrows = (long long)(g.gy + 2) * (g.gz + 2);
+    const int nsm = sm_count();
+    int best = 128;
+    double least = 1e300;
+    for (const auto &h : heights) {
+        const long long tiles = ntx * ((nrows + h.rows - 1) / h.rows);
+        const double t = (double)((tiles + nsm - 1) / nsm) * h.rows * h.per_row;
+        if (t < least) {
+            least = t;
+            best = h.rows;
+        }
+    }
+    return best;
+}
+
+// rows: 256-row tiles (one accumulator set), 64-128 rows (two), 0 = chosen
+// from the grid.  With two sets a tile's epilogue overlaps the next tile's MMAs; 256-row
 // tiles take fewer, larger MMAs per node (three N = 256 against two N = 256
 // and two N = 128 for the same products) and fewer stages, which outweighs
 // their epilogue running alone at 512 x 256 x 128 (tables and B image
@@ -725,12 +750,7 @@ int launch_am_contract_tc(const KernelArgs &a, const AmParams &m, void *stream, 
     const int ntx = (g.gx + TC_M - 1) / TC_M;
     const long long nrows = (long long)(g.gy + 2) * (g.gz + 2);
     const int nsm = sm_count();
-    if (rows == 0) {
-        // 256-row tiles when there are enough of them to keep every SM busy
-        // for two, else 128
-        const long long wide_tiles = (long long)ntx * ((nrows + 255) / 256);
-        rows = wide_tiles >= 2LL * nsm ? 256 : 128;
-    }
+    if (rows == 0) rows = am_default_rows(g);
     const bool wide = rows == 256;
     const int N = wide ? 256 : (rows >= 64 && rows <= 128 ? rows / 16 * 16 : 128);
     const long long ntiles = (long long)ntx * ((nrows + N - 1) / N);

@@ -2877,9 +2877,24 @@ static int pick_zchunk(const Geo &g, int tile_x)
     long long want = 148LL * 4;
     int zc = (int)((tiles * g.gz) / want);
     if (zc < 4) zc = 4;
-    if (zc > 32) zc = 32;
+    // (64-wide tiles: at most 8, which leaves more of them to run at once and
+    // finer ones to leave out; us per step, 8 / 16 / 32 planes: 256^3 FP64
+    // 218 / 223 / 244, FP32 139 / 140 / 149, 512 x 256 x 128 melt pool FP32
+    // 257 / 268 / 267)
+    if (zc > (tile_x > DTX ? 8 : 32)) zc = tile_x > DTX ? 8 : 32;
     if (zc > g.gz) zc = g.gz;
     return zc;
+}
+
+// Cells per thread before any tuning: two when 64 x 8 x 8 tiles still give
+// three CTAs to every SM, else one, whose smaller tiles keep a small domain's
+// latency down (us per step, one / two cells: 64^3 FP64 32 / 42; 317 x 149 x 83
+// melt pool FP32 147 / 129, 203 x 171 x 149 FP32 96 / 77, 256^3 FP64 230 / 218,
+// FP32 184 / 139, 512 x 256 x 128 melt pool FP32 365 / 257).
+int stencil_default_cpt(const Geo &g)
+{
+    const long long tiles = (long long)((g.gx + 63) / 64) * ((g.gy + DTY - 1) / DTY) * ((g.gz + 7) / 8);
+    return tiles >= 148 * 3 ? 2 : 1;
 }
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,

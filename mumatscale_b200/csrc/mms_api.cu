@@ -95,7 +95,7 @@ struct mms_ctx {
     mms_params p{};
     TmaHolder tma{};
     // FP32 AM contraction tile rows: 64-128 (a multiple of 16; two
-    // accumulator sets), 256 (one), 0 = 128; set by mms_set_am_tile or
+    // accumulator sets), 256 (one), 0 = chosen from the grid; set by mms_set_am_tile or
     // mms_autotune
     int am_rows = 0;
     // one timestep captured as a CUDA graph (kernel arguments only change
@@ -938,7 +938,7 @@ mms_status mms_autotune(mms_ctx *ctx, int reps, int *cells_per_thread, int *zchu
         }
     }
     // FP32 AM form: the contraction's tile (128-row tiles with two
-    // accumulator sets, or 256-row tiles with one), timed with the tables on
+    // accumulator sets, 256-row tiles with one, or the grid's default), timed with the tables on
     // shadows of the temperature and the layer flag; the tables are scratch
     // rebuilt by every step, and are rebuilt for the current step afterwards
     int am_rows = ctx->am_rows;
@@ -956,10 +956,11 @@ mms_status mms_autotune(mms_ctx *ctx, int reps, int *cells_per_thread, int *zchu
         if (sls) sa.d.lsindex = (int *)sls;
         const AmParams m = am_params(ctx->p);
         double best_am = 1e300;
-        const int am_cands[2] = {128, 256};
-        std::vector<float> am_ms[2];
+        constexpr int NC = 3;
+        const int am_cands[NC] = {128, 256, am_default_rows(g)};
+        std::vector<float> am_ms[NC];
         for (int r = 0; r < reps + 2; r++)
-            for (int ci = 0; ci < 2; ci++) {
+            for (int ci = 0; ci < NC; ci++) {
                 cudaEventRecord(e0, ctx->stream);
                 launch_temp_am(sa, m, ctx->prec, ctx->stream, nullptr, am_cands[ci]);
                 cudaEventRecord(e1, ctx->stream);
@@ -968,7 +969,7 @@ mms_status mms_autotune(mms_ctx *ctx, int reps, int *cells_per_thread, int *zchu
                 cudaEventElapsedTime(&t, e0, e1);
                 if (r >= 2) am_ms[ci].push_back(t);
             }
-        for (int ci = 0; ci < 2; ci++) {
+        for (int ci = 0; ci < NC; ci++) {
             std::sort(am_ms[ci].begin(), am_ms[ci].end());
             if (am_ms[ci][am_ms[ci].size() / 2] < best_am) {
                 best_am = am_ms[ci][am_ms[ci].size() / 2];
@@ -1384,7 +1385,12 @@ mms_status create_ctx(const mms_params *pin, int nslabs, int slab, mms_ctx **out
             (st = dalloc(ctx, &tm.act, (size_t)tiles)) || (p.am && (st = dalloc(ctx, &tm.am_max, 4 + 400 * (size_t)edges))))
             return fail(st);
     }
+    ctx->tma.cpt = stencil_default_cpt(g);
     if (set_tiles(ctx) != cudaSuccess) return fail(MMS_ERR_CUDA);
+    if (!ctx->tma.ok) {
+        ctx->tma.cpt = 1;
+        if (set_tiles(ctx) != cudaSuccess) return fail(MMS_ERR_CUDA);
+    }
     // orientation tables
     if (p.gnUseOrientation) {
         long long maxsites = 0;

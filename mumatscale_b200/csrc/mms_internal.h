@@ -287,6 +287,7 @@ int launch_step(const KernelArgs &a, const TmaHolder &tma, int precision, void *
 // and `on` are the caller's); tile_map_max: the most tiles, columns + rows +
 // layers of tiles any choice gives.
 void tile_geometry(KernelArgs &a, const TmaHolder &tma);
+int stencil_default_cpt(const Geo &g);
 void tile_map_max(const Geo &g, long long *tiles, long long *edges);
 // Builds the TMA descriptors of the stencil for the current buffers;
 // returns 0 when the driver cannot encode them (the stencil then uses its
@@ -328,11 +329,12 @@ struct AmParams {
 };
 // FP32 AM contraction on the tensor cores (am_tc.cu): tiles of 128 x cells
 // by `rows` (y, z) rows: 64-128 (two accumulator sets), 256 (one), or 0 =
-// 128.  The halo columns x = 0 and
+// chosen from the grid.  The halo columns x = 0 and
 // gx + 1 are filled only where they are read: launch_am_halo_fill writes
 // them into a temperature download buffer from the tables of the current
 // step (they are computed every step when the layer flag lsindex is kept).
 int launch_am_contract_tc(const KernelArgs &a, const AmParams &m, void *stream, int rows);
+int am_default_rows(const Geo &g);  // the rows that 0 stands for
 // the FP32 temperature as a tensor-store target (kernels.cu; map: a CUtensorMap)
 bool encode_t32_store(void *map, const KernelArgs &a, int bx, int by);
 int launch_am_halo_fill(const KernelArgs &a, const AmParams &m, double *dev_out, void *stream);
