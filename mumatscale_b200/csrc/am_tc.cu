@@ -672,11 +672,11 @@ __global__ void __launch_bounds__(256) k_am_halo(KernelArgs a, AmParams m, doubl
             acc = fmaf(__ldg(X + (long long)i * nx + xh), __ldg(Y + (long long)i * ny + J) * __ldg(Z + (long long)i * nz + K),
                        acc);
     const AmStep st = am_step(p, m, ts);
-    const long long cell = (long long)K * g.sz + (long long)J * g.sy + xh;
     const double T = zon[K] ? st.liniT + st.Tfront * (double)acc : 0.0;
     if (out) {
-        out[cell] = T;
+        out[(long long)K * g.rsz + (long long)J * g.rsy + xh] = T;  // the reference's layout
     } else {
+        const long long cell = (long long)K * g.sz + (long long)J * g.sy + xh;
         const float T32 = (float)T;
         a.d.T32[cell] = T32;
         if (a.d.lsindex && (double)T32 > p.Tliq) a.d.lsindex[cell] = 1;
@@ -775,10 +775,10 @@ int launch_am_contract_tc(const KernelArgs &a, const AmParams &m, void *stream, 
     return n;
 }
 
-int launch_am_halo_fill(const KernelArgs &a, const AmParams &m, double *dev_out, void *stream)
+int launch_am_halo_fill(const KernelArgs &a, const AmParams &m, double *ref_out, void *stream)
 {
     const long long e = 2LL * (a.g.gy + 2) * (a.g.gz + 2);
-    k_am_halo<<<(unsigned)((e + 255) / 256), 256, 0, (cudaStream_t)stream>>>(a, m, dev_out, 0);
+    k_am_halo<<<(unsigned)((e + 255) / 256), 256, 0, (cudaStream_t)stream>>>(a, m, ref_out, 0);
     return 1;
 }
 

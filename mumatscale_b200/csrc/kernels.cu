@@ -264,121 +264,138 @@ __global__ void k_am_tables(KernelArgs a, AmParams m)
     }
 }
 
-// T over tiles of (XL MX) x-cells by (G MY) (y, z) rows, G = 256 / XL: each
-// thread keeps MX x MY sums (x cells XL apart, MY consecutive rows), streaming
-// the node axis through shared memory 16 nodes at a time; per node a thread
-// reads MX X values (consecutive across the x lanes, no bank conflicts) and
-// MY YZ products (the same for the lanes of one row group) for MX MY fused
-// multiply-adds.
-template <typename Real>
-struct AmTile;
-template <>
-struct AmTile<double> {
-    static constexpr int XL = 16, MX = 4, MY = 8, MINB = 2;
-};
-template <>
-struct AmTile<float> {
-    static constexpr int XL = 16, MX = 4, MY = 8, MINB = 2;
-};
-constexpr int AMC_CH = 16, AMC_NT = 256;
+// T over tiles of 64 x cells by 128 (y, z) rows on the FP64 tensor cores (the
+// FP64 form's contraction; no 64-bit kind exists for tcgen05, whose FP32-form
+// kernel is in am_tc.cu).  Each of the eight warps keeps 32 x 32 sums as 4 x 4
+// tiles of mma.m8n8k4 (M: rows, N: x cells, K: nodes) and streams the node axis
+// through shared memory 16 nodes at a time: per four nodes eight 8-byte loads
+// feed sixteen products of 8 x 8 x 4.  The staging rows are padded by four
+// doubles, so that the 4 nodes x 4 cells of a half warp fall into sixteen
+// different banks.  Bounded by the FP64 pipe, which the tensor instruction fills
+// to 61 % (123 us at 251 x 127 x 67 under ncu); with scalar multiply-adds on the
+// same pipe it was 53 % busy.  With the tables: 251 x 127 x 67 117 -> 94 us, 512 x
+// 256 x 128 720 -> 549.  Two chunks in turn with one barrier each, or m16n8k8,
+// measured the same or slower (576, 598).
+constexpr int AMC_CH = 16, AMC_NT = 256, AMC_TX = 64, AMC_TR = 128;
 
-template <typename Real>
-__global__ void __launch_bounds__(AMC_NT, AmTile<Real>::MINB) k_am_contract(KernelArgs a, AmParams m)
+__device__ __forceinline__ void mma_f64(double (&c)[2], double a, double b)
 {
-    using TL = AmTile<Real>;
-    constexpr int XL = TL::XL, MX = TL::MX, MY = TL::MY, G = AMC_NT / XL;
-    constexpr int TX = XL * MX, TR = G * MY;
+    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+                 : "+d"(c[0]), "+d"(c[1])
+                 : "d"(a), "d"(b));
+}
+
+__device__ __forceinline__ void am_store(const KernelArgs &a, long long c, double T)
+{
+    a.d.T[c] = T;
+    if (a.d.lsindex && T > a.p.Tliq) a.d.lsindex[c] = 1;
+}
+
+__global__ void __launch_bounds__(AMC_NT, 2) k_am_contract(KernelArgs a, AmParams m, int apart)
+{
+    constexpr int SX = AMC_TX + 4, SR = AMC_TR + 4;
     const Ctl *ctl = a.d.ctl;
     if (stalled(ctl)) return;
     const Geo &g = a.g;
     const Phys &p = a.p;
     const int nx = g.gx + 2, ny = g.gy + 2, nz = g.gz + 2;
-    const Real *X = (const Real *)a.d.am_tab, *Y = X + (long long)AM_NT * nx, *Z = Y + (long long)AM_NT * ny;
+    const double *X = a.d.am_tab, *Y = X + (long long)AM_NT * nx, *Z = Y + (long long)AM_NT * ny;
     const int *zon = (const int *)(Z + (long long)AM_NT * nz);
-    __shared__ __align__(16) Real sX[AMC_CH][TX];
-    __shared__ __align__(16) Real sYZ[AMC_CH][TR];
-    const int tid = threadIdx.x, xl = tid % XL, grp = tid / XL;
-    const int x0 = blockIdx.x * TX;
-    const long long r0 = (long long)blockIdx.y * TR;  // row = K * ny + J
-    const long long nrows = (long long)ny * nz;
+    __shared__ __align__(16) double sX[AMC_CH][SX];
+    __shared__ __align__(16) double sYZ[AMC_CH][SR];
     __shared__ int s_any;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    // apart: tiles of interior x cells, the two halo columns apart
+    const int x0 = apart + blockIdx.x * AMC_TX, x1 = apart ? g.gx : g.gx + 1;
+    const long long r0 = (long long)blockIdx.y * AMC_TR;  // row = K * ny + J
+    const long long nrows = (long long)ny * nz;
+    if (apart && blockIdx.x == gridDim.x - 1) {
+        // a cell a thread
+        const long long row = r0 + tid % AMC_TR;
+        if (row >= nrows) return;
+        const int K = (int)(row / ny), J = (int)(row - (long long)K * ny), x = tid < AMC_TR ? 0 : nx - 1;
+        const bool on = zon[K] != 0;
+        double sum = 0.0;
+        if (on)
+#pragma unroll 8
+            for (int i = 0; i < AM_NT; i++)
+                sum = fma(X[(long long)i * nx + x], Y[(long long)i * ny + J] * Z[(long long)i * nz + K], sum);
+        const AmStep s = am_step(p, m, ctl->timestep + 1);
+        am_store(a, (long long)K * g.sz + (long long)J * g.sy + x, on ? s.liniT + s.Tfront * sum : 0.0);
+        return;
+    }
     if (tid == 0) s_any = 0;
     __syncthreads();
-    for (int q = tid; q < TR; q += AMC_NT)
-        if (r0 + q < nrows && zon[(r0 + q) / ny]) s_any = 1;
+    if (tid < AMC_TR && r0 + tid < nrows && zon[(r0 + tid) / ny]) s_any = 1;
     __syncthreads();
-    Real acc[MX][MY];
+    // this warp's 32 rows and 32 x cells of the tile, this lane's place in them
+    const int wr = (warp & 3) * 32, wx = (warp >> 2) * 32, lk = lane & 3, lm = lane >> 2;
+    double acc[4][4][2];
 #pragma unroll
-    for (int u = 0; u < MX; u++)
+    for (int u = 0; u < 4; u++)
 #pragma unroll
-        for (int q = 0; q < MY; q++) acc[u][q] = 0;
+        for (int v = 0; v < 4; v++) acc[u][v][0] = acc[u][v][1] = 0.0;
     if (s_any) {
-        // each thread stages the same x columns and (y, z) rows of every
-        // chunk: their table offsets are fixed for the whole sum
-        constexpr int XSTEP = AMC_NT / TX;
-        const int xx = tid % TX, xi0 = tid / TX;
-        const bool xin = x0 + xx < nx;
-        const Real *Xp = X + (x0 + xx);
-        static_assert(AMC_NT % TR == 0 || TR % AMC_NT == 0, "row staging");
-        constexpr int YSTEP = TR >= AMC_NT ? 1 : AMC_NT / TR;     // nodes apart
-        constexpr int RPT = TR >= AMC_NT ? TR / AMC_NT : 1;       // rows per thread
-        const int yi0 = TR >= AMC_NT ? 0 : tid / TR;
-        const Real *Yp[RPT];
-        const Real *Zp[RPT];
-        bool rin[RPT];
+        // each thread stages the same x column and (y, z) row of every chunk
+        const int xx = tid % AMC_TX, xi0 = tid / AMC_TX;
+        const bool xin = x0 + xx <= x1;
+        const double *Xp = X + (x0 + xx);
+        const int rl = tid % AMC_TR, yi0 = tid / AMC_TR;
+        const bool rin = r0 + rl < nrows;
+        const int Kr = rin ? (int)((r0 + rl) / ny) : 0, Jr = rin ? (int)(r0 + rl - (long long)Kr * ny) : 0;
+        const double *Yp = Y + Jr, *Zp = Z + Kr;
+        constexpr int XS = AMC_NT / AMC_TX, YS = AMC_NT / AMC_TR;  // nodes apart
+        constexpr int XN = AMC_CH / XS, YN = AMC_CH / YS;
+        // the next chunk's values are loaded while the current one is summed
+        double bx[XN], by[YN], bz[YN];
+        auto load = [&](int i0) {
 #pragma unroll
-        for (int w = 0; w < RPT; w++) {
-            const int rl = (tid % (TR < AMC_NT ? TR : AMC_NT)) + w * AMC_NT;
-            const long long row = r0 + rl;
-            rin[w] = row < nrows;
-            const int Kr = rin[w] ? (int)(row / ny) : 0, Jr = rin[w] ? (int)(row - (long long)Kr * ny) : 0;
-            Yp[w] = Y + Jr;
-            Zp[w] = Z + Kr;
-        }
+            for (int e = 0; e < XN; e++) bx[e] = xin ? Xp[(long long)(i0 + xi0 + XS * e) * nx] : 0.0;
+#pragma unroll
+            for (int e = 0; e < YN; e++) {
+                by[e] = rin ? Yp[(long long)(i0 + yi0 + YS * e) * ny] : 0.0;
+                bz[e] = rin ? Zp[(long long)(i0 + yi0 + YS * e) * nz] : 0.0;
+            }
+        };
+        load(0);
         for (int i0 = 0; i0 < AM_NT; i0 += AMC_CH) {
 #pragma unroll
-            for (int ii = xi0; ii < AMC_CH; ii += XSTEP)
-                sX[ii][xx] = xin ? Xp[(long long)(i0 + ii) * nx] : (Real)0;
+            for (int e = 0; e < XN; e++) sX[xi0 + XS * e][xx] = bx[e];
 #pragma unroll
-            for (int ii = yi0; ii < AMC_CH; ii += YSTEP)
-#pragma unroll
-                for (int w = 0; w < RPT; w++) {
-                    const int rl = (tid % (TR < AMC_NT ? TR : AMC_NT)) + w * AMC_NT;
-                    sYZ[ii][rl] = rin[w] ? Yp[w][(long long)(i0 + ii) * ny] * Zp[w][(long long)(i0 + ii) * nz]
-                                         : (Real)0;
-                }
+            for (int e = 0; e < YN; e++) sYZ[yi0 + YS * e][rl] = by[e] * bz[e];
             __syncthreads();
-#pragma unroll 4
-            for (int ii = 0; ii < AMC_CH; ii++) {
-                Real xv[MX], yz[MY];
+            if (i0 + AMC_CH < AM_NT) load(i0 + AMC_CH);
 #pragma unroll
-                for (int u = 0; u < MX; u++) xv[u] = sX[ii][xl + XL * u];
+            for (int k = 0; k < AMC_CH; k += 4) {
+                double fa[4], fb[4];
 #pragma unroll
-                for (int q = 0; q < MY; q++) yz[q] = sYZ[ii][grp * MY + q];
+                for (int u = 0; u < 4; u++) {
+                    fa[u] = sYZ[k + lk][wr + 8 * u + lm];
+                    fb[u] = sX[k + lk][wx + 8 * u + lm];
+                }
 #pragma unroll
-                for (int u = 0; u < MX; u++)
+                for (int u = 0; u < 4; u++)
 #pragma unroll
-                    for (int q = 0; q < MY; q++) acc[u][q] = fma(xv[u], yz[q], acc[u][q]);
+                    for (int v = 0; v < 4; v++) mma_f64(acc[u][v], fa[u], fb[v]);
             }
             __syncthreads();
         }
     }
     const AmStep s = am_step(p, m, ctl->timestep + 1);
 #pragma unroll
-    for (int q = 0; q < MY; q++) {
-        const long long row = r0 + grp * MY + q;
-        if (row >= nrows) break;
+    for (int u = 0; u < 4; u++) {
+        const long long row = r0 + wr + 8 * u + lm;
+        if (row >= nrows) continue;
         const int K = (int)(row / ny), J = (int)(row - (long long)K * ny);
         const bool on = zon[K] != 0;
+        const long long base = (long long)K * g.sz + (long long)J * g.sy;
 #pragma unroll
-        for (int u = 0; u < MX; u++) {
-            const int x = x0 + xl + XL * u;
-            if (x >= nx) continue;
-            const long long c = (long long)K * g.sz + (long long)J * g.sy + x;
-            const double T = on ? s.liniT + s.Tfront * (double)acc[u][q] : 0.0;
-            a.d.T[c] = T;
-            if (a.d.lsindex && T > p.Tliq) a.d.lsindex[c] = 1;
-        }
+        for (int v = 0; v < 4; v++)
+#pragma unroll
+            for (int e = 0; e < 2; e++) {
+                const int x = x0 + wx + 8 * v + 2 * lk + e;
+                if (x <= x1) am_store(a, base + x, on ? s.liniT + s.Tfront * acc[u][v][e] : 0.0);
+            }
     }
 }
 
@@ -2787,14 +2804,19 @@ __global__ void k_compute_d(KernelArgs a, double *out)
     out[c] = d;
 }
 
-__global__ void k_fill_temperature(KernelArgs a, double *out)
+// The temperature of every halo'd cell in the reference's layout, a block per
+// row of cells at a time.
+__global__ void k_fill_temperature(KernelArgs a, double *ref)
 {
-    const Ctl *ctl = a.d.ctl;
     const Geo &g = a.g;
-    long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (c >= g.N) return;
-    long long K = c / g.sz, J = (c % g.sz) / g.sy;
-    out[c] = temp_cell(a.p, a.d.T, a.d.T32, c, J, K, ctl->timestep);
+    const unsigned long long ts = a.d.ctl->timestep;
+    const long long rows = (long long)(g.gy + 2) * (g.gz + 2);
+    for (long long r = blockIdx.x; r < rows; r += gridDim.x) {
+        const int K = (int)(r / (g.gy + 2)), J = (int)(r - (long long)K * (g.gy + 2));
+        const long long c = (long long)K * g.sz + (long long)J * g.sy;
+        for (int i = threadIdx.x; i < g.rsy; i += blockDim.x)
+            ref[r * g.rsy + i] = temp_cell(a.p, a.d.T, a.d.T32, c + i, J, K, ts);
+    }
 }
 // Zero the entries of cells captured by the last step (list cells whose
 // capture produced a grain id): turns gr into the reference's ogr, and
@@ -3319,9 +3341,6 @@ int launch_temp_am(const KernelArgs &a, const AmParams &m, int precision, void *
     cudaStream_t st = (cudaStream_t)stream;
     const Geo &g = a.g;
     const long long tab = (long long)AM_NT * (g.gx + g.gy + g.gz + 6);  // the tiles' maxima are fewer
-    auto grid_of = [&](int tx, int tr) {
-        return dim3((unsigned)((g.gx + 2 + tx - 1) / tx), (unsigned)(((long long)(g.gy + 2) * (g.gz + 2) + tr - 1) / tr));
-    };
     int n = 1;
     PROF_BEGIN(KID_TEMP_AM);
     if (precision == MMS_PREC_F32) {
@@ -3329,9 +3348,14 @@ int launch_temp_am(const KernelArgs &a, const AmParams &m, int precision, void *
         k_am_tables<float><<<(unsigned)((tab + 255) / 256), 256, 0, st>>>(a, m);
         n += launch_am_contract_tc(a, m, st, rows);
     } else {
-        using T = AmTile<double>;
         k_am_tables<double><<<(unsigned)((tab + 255) / 256), 256, 0, st>>>(a, m);
-        k_am_contract<double><<<grid_of(T::XL * T::MX, AMC_NT / T::XL * T::MY), AMC_NT, 0, st>>>(a, m);
+        // the halo columns apart where they would cost another column of tiles
+        // (512 cells across: 0.574 -> 0.549 ms with the tables)
+        const int with = (g.gx + 2 + AMC_TX - 1) / AMC_TX, without = (g.gx + AMC_TX - 1) / AMC_TX;
+        const int apart = without < with ? 1 : 0;
+        const dim3 tiles((unsigned)with,  // (apart: the last column of CTAs is the halo's)
+                         (unsigned)(((long long)(g.gy + 2) * (g.gz + 2) + AMC_TR - 1) / AMC_TR));
+        k_am_contract<<<tiles, AMC_NT, 0, st>>>(a, m, apart);
         n++;
     }
     PROF_END(KID_TEMP_AM);
@@ -3482,11 +3506,10 @@ int launch_compute_d(const KernelArgs &a, int precision, double *dev_out, void *
     return 1;
 }
 
-int launch_fill_temperature(const KernelArgs &a, double *dev_out, void *stream)
+int launch_fill_temperature(const KernelArgs &a, double *ref_out, void *stream)
 {
-    cudaStream_t st = (cudaStream_t)stream;
-    int nb = (int)((a.g.N + 255) / 256);
-    k_fill_temperature<<<nb, 256, 0, st>>>(a, dev_out);
+    const long long rows = (long long)(a.g.gy + 2) * (a.g.gz + 2);
+    k_fill_temperature<<<(int)(rows < 148LL * 16 ? rows : 148LL * 16), 256, 0, (cudaStream_t)stream>>>(a, ref_out);
     return 1;
 }
 

@@ -1825,22 +1825,26 @@ mms_status mms_download(mms_ctx *ctx, mms_field field, void *host)
         }
         CU(copy_out(ctx, host, d.curv, sizeof(double)));
         return MMS_OK;
-    case MMS_FIELD_D:
-    case MMS_FIELD_TEMPERATURE: {
+    case MMS_FIELD_D: {
         double *tmp;
         if ((st = dalloc(ctx, &tmp, N))) return st;
-        if (field == MMS_FIELD_D) {
-            ctx->launches += launch_compute_d(ctx->ka, ctx->prec, tmp, ctx->stream);
-            ctx->launches += launch_mask_captured(ctx->ka, tmp, 1, ctx->stream);
-        } else {
-            ctx->launches += launch_fill_temperature(ctx->ka, tmp, ctx->stream);
-            // FP32 AM form: the halo columns, which no kernel of a step reads,
-            // from the tables of the current step
-            if (ctx->ka.p.temp_mode == 2 && ctx->prec == MMS_PREC_F32)
-                ctx->launches += launch_am_halo_fill(ctx->ka, am_params(ctx->p), tmp, ctx->stream);
-        }
+        ctx->launches += launch_compute_d(ctx->ka, ctx->prec, tmp, ctx->stream);
+        ctx->launches += launch_mask_captured(ctx->ka, tmp, 1, ctx->stream);
         CU(copy_out(ctx, host, tmp, sizeof(double)));
         dfree(ctx, tmp);
+        return MMS_OK;
+    }
+    case MMS_FIELD_TEMPERATURE: {
+        // straight into the staging buffer, in the caller's layout
+        double *stg = (double *)stage_buffer(ctx, (size_t)g.rN * sizeof(double));
+        if (!stg) return MMS_ERR_NOMEM;
+        ctx->launches += launch_fill_temperature(ctx->ka, stg, ctx->stream);
+        // FP32 AM form: the halo columns, which no kernel of a step reads,
+        // from the tables of the current step
+        if (ctx->ka.p.temp_mode == 2 && ctx->prec == MMS_PREC_F32)
+            ctx->launches += launch_am_halo_fill(ctx->ka, am_params(ctx->p), stg, ctx->stream);
+        CU(cudaMemcpyAsync(host, stg, (size_t)g.rN * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
+        CU(cudaStreamSynchronize(ctx->stream));
         return MMS_OK;
     }
     case MMS_FIELD_NUC_THRESHOLD: {

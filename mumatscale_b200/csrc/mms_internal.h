@@ -337,7 +337,7 @@ int launch_am_contract_tc(const KernelArgs &a, const AmParams &m, void *stream, 
 int am_default_rows(const Geo &g);  // the rows that 0 stands for
 // the FP32 temperature as a tensor-store target (kernels.cu; map: a CUtensorMap)
 bool encode_t32_store(void *map, const KernelArgs &a, int bx, int by);
-int launch_am_halo_fill(const KernelArgs &a, const AmParams &m, double *dev_out, void *stream);
+int launch_am_halo_fill(const KernelArgs &a, const AmParams &m, double *ref_out, void *stream);
 int am_tc_prepare();
 long long am_ximg_size(int gx, int gy, int gz);  // floats of a.d.am_ximg
 // Temperature of the next step for the AM model (tables + contraction);
@@ -358,7 +358,7 @@ int launch_fold_fs(const KernelArgs &a, long long nparts, void *stream, double *
 // pinned host memory through device-usable pointers; the caller
 // synchronises, after which both are current on the host.
 int launch_fold_fs_out(const KernelArgs &a, long long nparts, void *stream, double *host_sum, void *host_ctl);
-int launch_fill_temperature(const KernelArgs &a, double *dev_out, void *stream);
+int launch_fill_temperature(const KernelArgs &a, double *ref_out, void *stream);  // reference layout
 int launch_compute_d(const KernelArgs &a, int precision, double *dev_out, void *stream);
 int launch_repack(void *dst, long long dst_pitch, const void *src, long long src_pitch, int row_bytes, long long rows,
                   void *stream);
