@@ -920,7 +920,7 @@ def adjoint_workload(args) -> None:
 def ensemble_workload(args) -> None:
     """64 independent domains (edges from {32,48,64,96,128} per axis, cooling
     10-1000 K/s, nucleation 1e11-1e14 m^-3, seeded) in the FP32 form, stepped
-    as one batch (one graph per step, one persistent stencil launch, tile
+    as one batch (one graph per step, one stencil launch, tile
     autotuned) for 3000 steps; beside it (N=1) the same domains stepped one
     after another with mms_step.  Under torchrun the domains are dealt to
     the ranks by size (largest first to the least-loaded rank): no collective

@@ -562,7 +562,7 @@ class _BatchDomain(Domain):
 
 class Batch:
     """Many independent domains stepped together (mms_batch_*): one CUDA graph
-    per step with a single persistent stencil launch over all domains."""
+    per step with a single stencil launch over all domains."""
 
     def __init__(self, params: list, precision: int = PREC_F64, device: int = 0):
         arr = (Params * len(params))()
