@@ -2462,7 +2462,9 @@ __device__ __forceinline__ int capture_cell(const KernelArgs &a, const Real *fs,
 // 113,000 entries in flight, the others follow in a second round (256^3
 // directional deck with event timing: 13.2 us at 12,000 entries, 18.5 at
 // 58,000, 32.8 at 140,000; 14.3, 19.1 and 34.3 with 64-bit cell coordinates).
-// Four blocks an SM spill: 14.8, 20.7 and 31.9.
+// Four blocks an SM spill: 14.8, 20.7 and 31.9.  Longer lists are bounded by
+// throughput: 49 and 85 us after 1,500 and 2,600 steps, the same with four
+// blocks, 52 and 90 with the next entry and its slot fetched ahead.
 template <typename Real>
 __device__ __forceinline__ void capture_body(const KernelArgs &a, int bid, int nb)
 {
