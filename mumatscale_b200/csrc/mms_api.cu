@@ -2413,7 +2413,8 @@ mms_status batch_build_items(mms_batch *b);
 mms_status batch_refresh(mms_batch *b)
 {
     const size_t nd = b->doms.size(), ib = batch_item_bytes();
-    if (!b->items) return MMS_OK;
+    // after a rebuild that failed: tried again, nothing steps without it
+    if (!b->items) return batch_build_items(b);
     // a domain given a tile of its own returns to the batch's: the tile flags
     // and the stencil launch are sized for that one
     for (const mms_ctx *ctx : b->doms)
@@ -2442,8 +2443,16 @@ mms_status batch_refresh(mms_batch *b)
     return MMS_OK;
 }
 
+// The batch's items and tile flags for its tile.  The step graph holds both
+// addresses, so it goes first: a failure below leaves the batch with neither.
 mms_status batch_build_items(mms_batch *b)
 {
+    cudaStreamSynchronize(b->stream);
+    batch_drop_graph(b);
+    if (b->items) cudaFree(b->items);
+    if (b->act) cudaFree(b->act);
+    b->items = nullptr;
+    b->act = nullptr;
     const size_t ib = batch_item_bytes();
     std::vector<unsigned char> host(ib * b->doms.size());
     long long tiles = 0;
@@ -2458,28 +2467,25 @@ mms_status batch_build_items(mms_batch *b)
         drop_graph(ctx);
         tiles += ctx->ka.d.tm.n;
     }
-    if (b->items) cudaFree(b->items);
-    if (b->act) cudaFree(b->act);
-    b->items = nullptr;
-    b->act = nullptr;
     if (cudaMalloc(&b->act, (size_t)tiles) != cudaSuccess ||
         cudaMemsetAsync(b->act, 0, (size_t)tiles, b->stream) != cudaSuccess) {
+        cudaGetLastError();
         b->err = "cudaMalloc of the batch's tile flags failed";
         return MMS_ERR_NOMEM;
     }
     tiles = 0;
     for (size_t i = 0; i < b->doms.size(); i++)
         tiles += fill_batch_item(host.data() + ib * i, b->doms[i]->ka, b->doms[i]->tma, tiles, b->act);
+    b->total_tiles = tiles;
     if (cudaMalloc(&b->items, host.size()) != cudaSuccess) {
+        cudaGetLastError();
         b->err = "cudaMalloc of the batch items failed";
         return MMS_ERR_NOMEM;
     }
     if (cudaMemcpyAsync(b->items, host.data(), host.size(), cudaMemcpyHostToDevice, b->stream) != cudaSuccess ||
         cudaStreamSynchronize(b->stream) != cudaSuccess)
         return MMS_ERR_CUDA;
-    b->total_tiles = tiles;
     b->grid = batch_grid(b->prec, b->cpt);
-    batch_drop_graph(b);
     return batch_refresh(b);
 }
 

@@ -1,0 +1,80 @@
+"""Device memory as the library's host side holds it: mms_api.cu on a CUDA
+runtime in host memory (tests/host_runtime), which counts the memory held,
+refuses what does not fit and notes every use of memory already given back."""
+from __future__ import annotations
+
+import os
+import subprocess
+import sys
+from pathlib import Path
+
+import pytest
+
+ROOT = Path(__file__).resolve().parents[1]
+CSRC = ROOT / "mumatscale_b200" / "csrc"
+
+PRELUDE = """
+import ctypes as C
+import numpy as np
+import mumatscale_b200 as M
+lib = M.load_library()
+lib.host_runtime_held.restype = C.c_size_t
+lib.host_runtime_limit.argtypes = lib.host_runtime_total.argtypes = [C.c_size_t]
+lib.host_runtime_stale.restype = lib.host_runtime_graph_launches.restype = C.c_longlong
+held, limit, stale = lib.host_runtime_held, lib.host_runtime_limit, lib.host_runtime_stale
+ALL = 1 << 40
+p = M.read_deck(DECK)
+"""
+
+
+@pytest.fixture(scope="module")
+def run(tmp_path_factory):
+    """Runs a script on the library built with that runtime."""
+    lib = tmp_path_factory.mktemp("host_runtime") / "libmms_host.so"
+    sources = [CSRC / f for f in ("mms_api.cu", "host_setup.cpp", "deck.cpp", "output.cpp")]
+    sources.append(ROOT / "tests" / "host_runtime" / "host_runtime.cpp")
+    subprocess.run(["g++", "-x", "c++", "-std=c++17", "-O1", "-fPIC", "-shared", "-w", "-I/usr/local/cuda/include",
+                    f"-I{CSRC}", "-o", str(lib), *map(str, sources), "-lz", "-ldl", "-lpthread", "-Wl,--no-undefined"],
+                   check=True)
+    deck = ROOT / "tests" / "golden" / "decks" / "small4.in"
+
+    def go(script: str) -> str:
+        r = subprocess.run([sys.executable, "-c", f"from pathlib import Path\nDECK = Path({str(deck)!r})" + PRELUDE + script],
+                           cwd=ROOT, env=dict(os.environ, MMS_LIBRARY=str(lib)), capture_output=True, text=True)
+        assert r.returncode == 0, r.stdout + r.stderr
+        return r.stdout
+
+    return go
+
+
+@pytest.mark.parametrize("spare", [0, 1, 2, 3])
+def test_batch_after_a_rebuild_without_memory(run, spare):
+    """A tile whose buffers do not fit: the batch steps no more until they do,
+    and never with those it gave back (spare: the buffers that still fit)."""
+    run(f"""
+with M.Batch([p, p]) as b:
+    b.step(3)
+    before = held()
+    # what a rebuild gives back: measured by one that fails at once
+    limit(0)
+    try:
+        b.set_stencil_tile(2, 1)
+        raise SystemExit("no failure")
+    except M.MmsError as e:
+        assert e.status == 11, e
+    freed = before - held()
+    assert freed > 0
+    limit(held() + {spare} * freed // 4)
+    try:
+        b.step(2)
+        done = 2
+    except M.MmsError as e:
+        assert e.status == 11, e
+        done = 0
+    assert [d.timestep for d in b.domains] == [3 + done] * 2
+    limit(ALL)
+    b.step(4)
+    assert [d.timestep for d in b.domains] == [7 + done] * 2
+    assert b.stencil_tile()[:2] == (2, 1)
+assert stale() == 0, stale()
+""")
