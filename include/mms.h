@@ -543,7 +543,9 @@ mms_status mms_adjoint_record(mms_ctx *ctx, int nsteps, int checkpoint_every);
  * (FP64).  Each segment between checkpoints is recomputed from its
  * checkpoint by frozen replay, then differentiated backwards.  The work
  * buffers (checkpoint_every states, two sets of adjoints) are made by the
- * first call and kept until the record is released or replaced. */
+ * first call.  Up to 4 GiB of them stay with the record until it is released
+ * or replaced, or until an allocation of this library does not fit beside
+ * them; larger ones are given back at the end of the call. */
 mms_status mms_adjoint_gradient(mms_ctx *ctx, const double *target_ce, mms_adjoint_result *out);
 /* Loss of the frozen replay of the whole recorded run from its first
  * checkpoint with Dliq, part_coef and GibbsThomsonCoef multiplied by

@@ -184,11 +184,13 @@ struct mms_ctx {
         unsigned char *flags = nullptr;  // nrec x N
         double *curv = nullptr;          // nrec x N (TipCurvature)
         char *ckpt = nullptr;            // nckpt x 3 x N x element size
-        // work buffers of the gradient and the replayed loss, made by the
-        // first of them and kept as long as the record
-        char *seg = nullptr;             // seg_states x 3 x N: replayed states, halos as recorded
-        long long seg_states = 0;        // 2 for the loss, at least `every` for the gradient
-        char *lam = nullptr;             // 6 x N: adjoints of (ce, cl, fs), two sets
+        // work buffers of the gradient and the replayed loss (adj_buffers),
+        // parts of one allocation that is not among `allocs`
+        char *work = nullptr;
+        size_t work_bytes = 0;
+        long long states = 0;            // replayed states: 2 for the loss, at least `every` for the gradient
+        char *seg = nullptr;             // states x 3 x N, halos as recorded
+        char *lam = nullptr;             // 6 x N: adjoints of (ce, cl, fs), two sets (gradient only)
         double *tgt = nullptr;           // N
         double *partial = nullptr;       // adj_nblocks x ADJ_SLOTS
         double *acc = nullptr;           // ADJ_SLOTS gradient sums, then the loss
@@ -206,12 +208,72 @@ namespace {
         }                                                                               \
     } while (0)
 
+// Contexts whose adjoint work buffers lie idle between two calls.  Only the
+// thread that holds the lock may free those of a context in the list; a
+// context leaves it before its buffers are used or dropped.
+struct IdleWork {
+    std::mutex mu;
+    std::vector<mms_ctx *> of;
+};
+IdleWork &idle_work()
+{
+    static IdleWork *w = new IdleWork();  // outlives every context
+    return *w;
+}
+
+void adj_drop_work(mms_ctx *ctx)
+{
+    mms_ctx::AdjRec &r = ctx->adj;
+    if (r.work) cudaFree(r.work);
+    r.work = r.seg = r.lam = nullptr;
+    r.tgt = r.partial = r.acc = nullptr;
+    r.work_bytes = 0;
+    r.states = 0;
+}
+
+void adj_claim_work(mms_ctx *ctx)
+{
+    IdleWork &w = idle_work();
+    std::lock_guard<std::mutex> lock(w.mu);
+    w.of.erase(std::remove(w.of.begin(), w.of.end(), ctx), w.of.end());
+}
+
+}  // namespace
+
+// cudaMalloc on the current device; where memory is short, idle work buffers
+// of any context on it are given back and it is tried again.  A failure leaves no
+// error behind for the next launch check to find.
+int mms::device_malloc(void **p, size_t bytes)
+{
+    cudaError_t e = cudaMalloc(p, bytes);
+    if (e == cudaSuccess) return e;
+    cudaGetLastError();
+    if (e != cudaErrorMemoryAllocation) return e;
+    int dev = 0;
+    cudaGetDevice(&dev);
+    IdleWork &w = idle_work();
+    std::lock_guard<std::mutex> lock(w.mu);
+    bool any = false;
+    for (size_t i = 0; i < w.of.size();)
+        if (w.of[i]->device == dev) {
+            adj_drop_work(w.of[i]);
+            w.of.erase(w.of.begin() + (long)i);
+            any = true;
+        } else {
+            i++;
+        }
+    if (any && (e = cudaMalloc(p, bytes)) != cudaSuccess) cudaGetLastError();
+    return e;
+}
+
+namespace {
+
 template <typename T>
 mms_status dalloc(mms_ctx *ctx, T **ptr, size_t count, bool zero = true)
 {
     void *p = nullptr;
     size_t bytes = sizeof(T) * (count ? count : 1);
-    cudaError_t e = cudaMalloc(&p, bytes);
+    cudaError_t e = (cudaError_t)device_malloc(&p, bytes);
     if (e != cudaSuccess) {
         ctx->err = std::string("cudaMalloc: ") + cudaGetErrorString(e);
         return MMS_ERR_NOMEM;
@@ -855,7 +917,7 @@ mms_status mms_autotune(mms_ctx *ctx, int reps, int *cells_per_thread, int *zchu
     // es > 0: a field, placed as dalloc_field places it (es = its element size)
     auto shadow_of = [&](const void *src, size_t bytes, void **dst, size_t es = 0) -> cudaError_t {
         void *raw = nullptr;
-        cudaError_t e = cudaMalloc(&raw, bytes + (es ? 16 : 0));
+        cudaError_t e = (cudaError_t)device_malloc(&raw, bytes + (es ? 16 : 0));
         if (e != cudaSuccess) return e;
         shadow.push_back(raw);
         *dst = es ? (void *)((char *)raw + 16 - es) : raw;
@@ -1492,6 +1554,8 @@ mms_status mms_destroy(mms_ctx *ctx)
     if (ctx->stream) cudaStreamSynchronize(ctx->stream);
     for (void *p : ctx->allocs) cudaFree(p);
     ctx->allocs.clear();
+    adj_claim_work(ctx);
+    adj_drop_work(ctx);
     for (cudaEvent_t e : ctx->slab_events) cudaEventDestroy(e);
     ctx->slab_events.clear();
     nccl_release(ctx);
@@ -2127,11 +2191,8 @@ void adj_free(mms_ctx *ctx)
     dfree(ctx, ctx->adj.flags);
     dfree(ctx, ctx->adj.curv);
     dfree(ctx, ctx->adj.ckpt);
-    dfree(ctx, ctx->adj.seg);
-    dfree(ctx, ctx->adj.lam);
-    dfree(ctx, ctx->adj.tgt);
-    dfree(ctx, ctx->adj.partial);
-    dfree(ctx, ctx->adj.acc);
+    adj_claim_work(ctx);
+    adj_drop_work(ctx);
     ctx->adj = mms_ctx::AdjRec{};
 }
 
@@ -2149,35 +2210,70 @@ mms_status adj_save_ckpt(mms_ctx *ctx, long long idx, unsigned long long ts)
     return MMS_OK;
 }
 
-// The work buffers of the record.  Allocated on the first call (128^3 FP64,
-// checkpoints every 50 steps: 2.6 GB, whose allocation, clearing and release
-// took about as long as the gradient itself when each call did them); the
-// replay writes interior cells, and no halo cell changes during a run, so the
-// states' halos are filled here once instead of copying the checkpoint into
-// every state.
+// The work buffers of a gradient (or of the replayed loss alone), for the
+// duration of a call: made by the first, in one piece; afterwards they stay with
+// the record while they are no larger than ADJ_KEEP and no allocation of the
+// library needs their memory (device_malloc), and larger ones go at the end of
+// the call.  (128^3 FP64, checkpoints every 50 steps: 2.8 GB, whose allocation,
+// clearing and release took about as long as the gradient itself when each call
+// did them.)  The replay writes interior cells, and no halo cell changes during a
+// run, so the states' halos are filled here once instead of copying the
+// checkpoint into every state.
+constexpr size_t ADJ_KEEP = (size_t)4 << 30;
+
+struct AdjWork {
+    mms_ctx *ctx;
+    explicit AdjWork(mms_ctx *c) : ctx(c) { adj_claim_work(ctx); }
+    ~AdjWork()
+    {
+        if (!ctx->adj.work) return;
+        cudaStreamSynchronize(ctx->stream);
+        if (ctx->adj.work_bytes > ADJ_KEEP) {
+            adj_drop_work(ctx);
+            return;
+        }
+        IdleWork &w = idle_work();
+        std::lock_guard<std::mutex> lock(w.mu);
+        w.of.push_back(ctx);
+    }
+    AdjWork(const AdjWork &) = delete;
+    AdjWork &operator=(const AdjWork &) = delete;
+};
+
 mms_status adj_buffers(mms_ctx *ctx, bool gradient)
 {
     mms_ctx::AdjRec &r = ctx->adj;
     const Geo &g = ctx->ka.g;
     const size_t N = (size_t)g.N, es = elem_size(ctx);
     const long long states = gradient ? std::max(2, r.every) : 2;
-    mms_status st = MMS_OK;
-    if (r.seg_states < states) {
-        CU(cudaStreamSynchronize(ctx->stream));
-        dfree(ctx, r.seg);
-        r.seg = nullptr;
-        r.seg_states = 0;
-        if ((st = dalloc(ctx, &r.seg, (size_t)states * 3 * N * es, false))) return st;
-        r.seg_states = states;
-        for (long long s = 0; s < states; s++)
-            CU(cudaMemcpyAsync(state_slot(r.seg, s, 0, N, es), state_slot(r.ckpt, 0, 0, N, es), 3 * N * es,
-                               cudaMemcpyDeviceToDevice, ctx->stream));
+    if (r.states >= states && (r.lam || !gradient)) return MMS_OK;
+    CU(cudaStreamSynchronize(ctx->stream));
+    adj_drop_work(ctx);
+    size_t bytes = 0;
+    auto part = [&](size_t n) {
+        const size_t at = bytes;
+        bytes += (n + 255) / 256 * 256;
+        return at;
+    };
+    const size_t seg = part((size_t)states * 3 * N * es), lam = part(gradient ? 6 * N * es : 0),
+                 tgt = part(N * sizeof(double)), partial = part((size_t)adj_nblocks(g) * ADJ_SLOTS * sizeof(double)),
+                 acc = part((ADJ_SLOTS + 1) * sizeof(double));
+    const cudaError_t e = (cudaError_t)device_malloc((void **)&r.work, bytes);
+    if (e != cudaSuccess) {
+        ctx->err = std::string("cudaMalloc: ") + cudaGetErrorString(e);
+        return MMS_ERR_NOMEM;
     }
-    auto need = [&](auto **ptr, size_t n) { return *ptr ? MMS_OK : dalloc(ctx, ptr, n, false); };
-    if ((st = need(&r.tgt, N)) || (st = need(&r.partial, (size_t)adj_nblocks(g) * ADJ_SLOTS)) ||
-        (st = need(&r.acc, ADJ_SLOTS + 1)))
-        return st;
-    return gradient ? need(&r.lam, 6 * N * es) : MMS_OK;
+    r.work_bytes = bytes;
+    r.seg = r.work + seg;
+    if (gradient) r.lam = r.work + lam;
+    r.tgt = (double *)(r.work + tgt);
+    r.partial = (double *)(r.work + partial);
+    r.acc = (double *)(r.work + acc);
+    for (long long s = 0; s < states; s++)
+        CU(cudaMemcpyAsync(state_slot(r.seg, s, 0, N, es), state_slot(r.ckpt, 0, 0, N, es), 3 * N * es,
+                           cudaMemcpyDeviceToDevice, ctx->stream));
+    r.states = states;
+    return MMS_OK;
 }
 
 // Phys with Dliq, part_coef and the Gibbs-Thomson coefficient scaled, each
@@ -2268,6 +2364,7 @@ mms_status mms_adjoint_replay_loss(mms_ctx *ctx, const double *target_ce, const 
     const size_t N = (size_t)g.N, es = elem_size(ctx);
     const mms_ctx::AdjRec &r = ctx->adj;
     const Phys ph = scaled_phys(ctx, scale);
+    AdjWork work(ctx);
     mms_status st = adj_buffers(ctx, false);
     if (st) return st;
     cudaError_t e = copy_in(ctx, r.tgt, target_ce, sizeof(double));
@@ -2308,6 +2405,7 @@ mms_status mms_adjoint_gradient(mms_ctx *ctx, const double *target_ce, mms_adjoi
     const size_t N = (size_t)g.N, es = elem_size(ctx);
     const mms_ctx::AdjRec &r = ctx->adj;
     const Phys &ph = ctx->ka.p;
+    AdjWork work(ctx);
     mms_status st = adj_buffers(ctx, true);
     if (st) return st;
     cudaError_t e = copy_in(ctx, r.tgt, target_ce, sizeof(double));
@@ -2427,7 +2525,7 @@ mms_status batch_refresh(mms_batch *b)
         tiles += fill_batch_item(host.data() + ib * i, ctx->ka, ctx->tma, tiles, b->act);
         for (int w = 0; w < 4; w++) begin[w * (nd + 1) + i + 1] = begin[w * (nd + 1) + i] + batch_blocks(ctx->ka, w);
     }
-    if (!b->begin && cudaMalloc(&b->begin, sizeof(int) * begin.size()) != cudaSuccess) {
+    if (!b->begin && device_malloc((void **)&b->begin, sizeof(int) * begin.size()) != cudaSuccess) {
         b->err = "cudaMalloc of the batch prefixes failed";
         return MMS_ERR_NOMEM;
     }
@@ -2467,9 +2565,8 @@ mms_status batch_build_items(mms_batch *b)
         drop_graph(ctx);
         tiles += ctx->ka.d.tm.n;
     }
-    if (cudaMalloc(&b->act, (size_t)tiles) != cudaSuccess ||
+    if (device_malloc((void **)&b->act, (size_t)tiles) != cudaSuccess ||
         cudaMemsetAsync(b->act, 0, (size_t)tiles, b->stream) != cudaSuccess) {
-        cudaGetLastError();
         b->err = "cudaMalloc of the batch's tile flags failed";
         return MMS_ERR_NOMEM;
     }
@@ -2477,8 +2574,7 @@ mms_status batch_build_items(mms_batch *b)
     for (size_t i = 0; i < b->doms.size(); i++)
         tiles += fill_batch_item(host.data() + ib * i, b->doms[i]->ka, b->doms[i]->tma, tiles, b->act);
     b->total_tiles = tiles;
-    if (cudaMalloc(&b->items, host.size()) != cudaSuccess) {
-        cudaGetLastError();
+    if (device_malloc(&b->items, host.size()) != cudaSuccess) {
         b->err = "cudaMalloc of the batch items failed";
         return MMS_ERR_NOMEM;
     }
@@ -2742,7 +2838,7 @@ mms_status mms_batch_autotune(mms_batch *b, int reps, int *cells_per_thread, int
         // es > 0: a field, placed as dalloc_field places it
         auto sh = [&](const void *src, size_t bytes, size_t es = 0) -> void * {
             void *raw = nullptr;
-            if (cudaMalloc(&raw, bytes + (es ? 16 : 0)) != cudaSuccess) return nullptr;
+            if (device_malloc(&raw, bytes + (es ? 16 : 0)) != cudaSuccess) return nullptr;
             shadow.push_back(raw);
             void *d = es ? (void *)((char *)raw + 16 - es) : raw;
             cudaMemcpyAsync(d, src, bytes, cudaMemcpyDeviceToDevice, b->stream);
@@ -2770,7 +2866,7 @@ mms_status mms_batch_autotune(mms_batch *b, int reps, int *cells_per_thread, int
     const size_t ib = batch_item_bytes();
     std::vector<unsigned char> host(ib * nd);
     void *ditems = nullptr;
-    if (cudaMalloc(&ditems, host.size()) != cudaSuccess) {
+    if (device_malloc(&ditems, host.size()) != cudaSuccess) {
         release();
         return MMS_ERR_NOMEM;
     }

@@ -261,6 +261,10 @@ enum KernelId : int {
     KID_TEMP_AM = 0, KID_NUC, KID_ACT, KID_CURV, KID_DIFFUSE_FS, KID_LIST, KID_CAPTURE, KID_COUNT
 };
 
+// cudaMalloc (mms_api.cu) that gives idle buffers of the library's contexts
+// back where memory is short; returns the cudaError_t.
+int device_malloc(void **p, size_t bytes);
+
 // Opaque storage for the stencil's TMA descriptors (built in kernels.cu).
 struct TmaHolder {
     alignas(128) unsigned char bytes[6 * 128];

@@ -181,10 +181,10 @@ int site_draw_device(const SiteDrawArgs &args, const std::vector<double> &pv, co
         if (e == cudaSuccess && x != cudaSuccess) e = x;
         return e == cudaSuccess;
     };
+    auto room = [&](auto **p, size_t n) { return chk((cudaError_t)device_malloc((void **)p, n * sizeof **p)); };
     const size_t np = preset_q.size() ? preset_q.size() : 1;
-    if (chk(cudaMalloc(&dpv, pv.size() * sizeof(double))) && chk(cudaMalloc(&dps, ps.size() * sizeof(double))) &&
-        chk(cudaMalloc(&dpq, np * sizeof(long long))) && chk(cudaMalloc(&dpt, np * sizeof(float))) &&
-        chk(cudaMalloc(&dcnt, (size_t)nblk * sizeof(int))) && chk(cudaMalloc(&doff, (size_t)nblk * sizeof(long long))) &&
+    if (room(&dpv, pv.size()) && room(&dps, ps.size()) && room(&dpq, np) && room(&dpt, np) &&
+        room(&dcnt, (size_t)nblk) && room(&doff, (size_t)nblk) &&
         chk(cudaMemcpy(dpv, pv.data(), pv.size() * sizeof(double), cudaMemcpyHostToDevice)) &&
         chk(cudaMemcpy(dps, ps.data(), ps.size() * sizeof(double), cudaMemcpyHostToDevice)) &&
         (preset_q.empty() ||
@@ -198,8 +198,7 @@ int site_draw_device(const SiteDrawArgs &args, const std::vector<double> &pv, co
             for (long long b = 0; b < nblk; b++) off[b] = tot, tot += cnt[b];
             const size_t nt = tot ? (size_t)tot : 1;
             if (chk(cudaMemcpy(doff, off.data(), off.size() * sizeof(long long), cudaMemcpyHostToDevice)) &&
-                chk(cudaMalloc(&dcell, nt * sizeof(long long))) && chk(cudaMalloc(&dthr, nt * sizeof(float))) &&
-                chk(cudaMalloc(&drank, nt * sizeof(int)))) {
+                room(&dcell, nt) && room(&dthr, nt) && room(&drank, nt)) {
                 k_site_write<<<(unsigned)nblk, SD_NT>>>(a, dpv, dps, dpq, dpt, doff, dcell, dthr, drank);
                 cells.resize((size_t)tot);
                 thr.resize((size_t)tot);

@@ -5,6 +5,7 @@
 // test_host_memory.py).  Steps only count; no field changes.
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <cstring>
 #include <functional>
 #include <map>
@@ -21,14 +22,14 @@ namespace {
 std::mutex mu;
 std::map<const char *, size_t> live;  // device allocations
 size_t held = 0, limit = (size_t)1 << 40, total = (size_t)1 << 40;
-long long stale = 0;     // uses of memory that is not allocated
-long long launched = 0;  // graph launches
-cudaError_t last = cudaSuccess;
+std::atomic<long long> stale{0};  // uses of memory that is not allocated
+std::atomic<long long> launched{0};  // graph launches
+thread_local cudaError_t last = cudaSuccess;
 
 struct Graph {
     std::vector<std::function<void()>> work;
 };
-Graph *capturing = nullptr;
+thread_local Graph *capturing = nullptr;
 
 bool valid(const void *p)
 {
@@ -108,6 +109,7 @@ cudaError_t cudaGetDeviceProperties(cudaDeviceProp *p, int)
     p->totalGlobalMem = total;
     return cudaSuccess;
 }
+cudaError_t cudaGetDevice(int *d) { *d = 0; return cudaSuccess; }
 cudaError_t cudaSetDevice(int) { return cudaSuccess; }
 cudaError_t cudaDeviceEnablePeerAccess(int, unsigned) { return cudaSuccess; }
 const char *cudaGetErrorString(cudaError_t e) { return e == cudaErrorMemoryAllocation ? "out of memory" : "error"; }
@@ -116,7 +118,7 @@ cudaError_t cudaMemcpyAsync(void *d, const void *s, size_t n, cudaMemcpyKind k, 
 {
     if ((k == cudaMemcpyHostToDevice || k == cudaMemcpyDeviceToDevice) && !valid(d)) { stale++; return cudaSuccess; }
     if ((k == cudaMemcpyDeviceToHost || k == cudaMemcpyDeviceToDevice) && !valid(s)) { stale++; return cudaSuccess; }
-    std::memcpy(d, s, n);
+    if (k != cudaMemcpyDeviceToDevice) std::memcpy(d, s, n);  // (no field's values matter here)
     return cudaSuccess;
 }
 cudaError_t cudaMemcpyPeerAsync(void *d, int, const void *s, int, size_t n, cudaStream_t)

@@ -78,3 +78,104 @@ with M.Batch([p, p]) as b:
     assert b.stencil_tile()[:2] == (2, 1)
 assert stale() == 0, stale()
 """)
+
+
+RECORD = """
+d = M.Domain(p)
+d.step(4)
+target = d.download("ce")
+def record(steps, every):
+    d.adjoint_record(steps, every)
+    return held()
+def tight(fn, *args):
+    try:
+        fn(*args)
+    except M.MmsError as e:
+        assert e.status == 11, e
+        return True
+"""
+
+
+def test_a_second_domain_fits_after_a_gradient(run):
+    """What fitted beside a record before its gradient fits after it."""
+    run(RECORD + """
+before = record(20, 10)
+g = d.adjoint_gradient(target)
+kept = held() - before
+assert kept > 0
+for make in (lambda: M.Domain(p), lambda: M.Batch([p])):
+    with make():  # its own size, measured with room to spare
+        size = held() - before - kept
+    d.adjoint_gradient(target)
+    assert held() == before + kept
+    limit(before + size)
+    with make():
+        pass
+    limit(ALL)
+    assert held() == before  # the buffers went
+    assert d.adjoint_gradient(target) == g
+    assert d.adjoint_replay_loss(target) == g["loss"]
+    assert held() == before + kept
+d.adjoint_release()
+d.close()
+assert held() == 0 and stale() == 0
+""")
+
+
+def test_large_work_buffers_go_with_the_call(run):
+    run(RECORD + """
+state = 3 * 8 * d.num_cells()
+before = record(3, (5 << 30) // state)  # states of 5 GiB
+d.adjoint_gradient(target)
+assert held() == before
+d.adjoint_replay_loss(target)  # two states
+assert 0 < held() - before < 1 << 30
+assert stale() == 0
+""")
+
+
+def test_a_gradient_without_memory(run):
+    """It fails with the status it always had, holds nothing, and both the
+    record and the domain go on."""
+    run(RECORD + """
+before = record(20, 10)
+limit(before + 1000)
+assert tight(d.adjoint_gradient, target)
+assert tight(d.adjoint_replay_loss, target)
+assert held() == before
+d.step(3)
+limit(ALL)
+assert d.adjoint_gradient(target)["steps"] == 20
+d.adjoint_record(5, 5)
+assert d.adjoint_gradient(target)["steps"] == 5
+assert stale() == 0
+""")
+
+
+def test_buffers_are_given_back_between_threads(run):
+    """One thread differentiates while another makes domains that fit only
+    beside idle buffers that are given back."""
+    run(RECORD + """
+import threading
+before = record(20, 10)
+d.adjoint_gradient(target)
+kept = held() - before
+with M.Domain(p):
+    size = held() - before - kept
+limit(before + kept // 2 + size)
+stop, made = threading.Event(), 0
+def differentiate():
+    while not stop.is_set():
+        tight(d.adjoint_gradient, target)
+t = threading.Thread(target=differentiate)
+t.start()
+for _ in range(40):
+    if not tight(lambda: M.Domain(p).close()):
+        made += 1
+stop.set()
+t.join()
+limit(ALL)
+assert d.adjoint_gradient(target)["steps"] == 20
+d.close()
+assert stale() == 0 and held() == 0
+""")
