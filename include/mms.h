@@ -302,6 +302,10 @@ mms_status mms_set_site_orientations(mms_ctx *ctx, int64_t n, const int32_t *gxy
  * usable.  block = -1 turns the hook off.  The context is in error after such
  * a step; destroy it. */
 mms_status mms_test_hold_list_block(mms_ctx *ctx, int block, unsigned polls);
+/* Test hook: the stencil tiles of the domain's tile map (0: it has none, and
+ * every step visits the whole domain), and how many of them the last step left
+ * out as being at rest. */
+mms_status mms_test_tile_map(mms_ctx *ctx, int *tiles, int *left_out);
 
 /* A pre-filled microstructure (for example a substrate of columnar grains):
  * defines grains 1..n with the given row-major rotation matrices, so that

@@ -170,6 +170,7 @@ def load_library(build_if_missing: bool = True) -> C.CDLL:
         "mms_params_free_lists": (None, [C.POINTER(Params)]),
         "mms_params_size": (C.c_size_t, []),
         "mms_test_hold_list_block": (I, [P, I, C.c_uint]),
+        "mms_test_tile_map": (I, [P, C.POINTER(I), C.POINTER(I)]),
         "mms_slab_nccl_unique_id": (I, [C.c_char_p, P]),
         "mms_slab_nccl_init": (I, [P, C.c_char_p, P]),
         "mms_slab_nccl_step": (I, [P, I]),
@@ -519,6 +520,13 @@ class Domain:
         next step on, list block `block` publishes no status word and the
         look-back waits give up after `polls` polls (-1: off)."""
         _check(_lib().mms_test_hold_list_block(self._ctx, block, polls), "mms_test_hold_list_block", self._ctx)
+
+    def test_tile_map(self) -> tuple[int, int]:
+        """Test hook (mms_test_tile_map): the tiles of the domain's tile map
+        (0: none) and how many of them the last step left out."""
+        n, out = C.c_int(), C.c_int()
+        _check(_lib().mms_test_tile_map(self._ctx, C.byref(n), C.byref(out)), "mms_test_tile_map", self._ctx)
+        return n.value, out.value
 
     def set_grains(self, rotmats: np.ndarray) -> None:
         """Grains 1..n of a pre-filled microstructure (row-major 3x3 rotations)."""

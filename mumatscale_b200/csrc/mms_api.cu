@@ -138,6 +138,7 @@ struct mms_ctx {
     uint64_t launches = 0;
     bool stepped = false;
     bool batched = false;  // stepped by an mms_batch
+    const unsigned char *batch_act = nullptr;  // this domain's part of its tile flags
     std::string err;
     size_t bytes = 0;
     std::vector<void *> allocs;
@@ -1582,6 +1583,20 @@ mms_status mms_test_hold_list_block(mms_ctx *ctx, int block, unsigned polls)
     return MMS_OK;
 }
 
+mms_status mms_test_tile_map(mms_ctx *ctx, int *tiles, int *left_out)
+{
+    if (!ctx || !tiles || !left_out) return MMS_ERR_ARG;
+    cudaSetDevice(ctx->device);
+    const TileMap &tm = ctx->ka.d.tm;
+    *tiles = tm.on ? tm.n : 0;
+    *left_out = 0;
+    if (!tm.on) return MMS_OK;
+    std::vector<unsigned char> act((size_t)tm.n);
+    CU(d2h(ctx, act.data(), ctx->batch_act ? ctx->batch_act : tm.act, act.size()));
+    for (unsigned char v : act) *left_out += !v;
+    return MMS_OK;
+}
+
 mms_status mms_set_grains(mms_ctx *ctx, int n, const double *rotmat9)
 {
     if (!ctx || n < 0 || (n && !rotmat9)) return MMS_ERR_ARG;
@@ -2558,6 +2573,7 @@ mms_status batch_build_items(mms_batch *b)
         mms_ctx *ctx = b->doms[i];
         ctx->tma.cpt = b->cpt;
         ctx->tma.zc = b->zc;
+        ctx->batch_act = nullptr;
         if (set_tiles(ctx) != cudaSuccess || !ctx->tma.ok) {
             b->err = "TMA descriptors could not be encoded for a batched domain";
             return MMS_ERR_CUDA;
@@ -2571,8 +2587,10 @@ mms_status batch_build_items(mms_batch *b)
         return MMS_ERR_NOMEM;
     }
     tiles = 0;
-    for (size_t i = 0; i < b->doms.size(); i++)
+    for (size_t i = 0; i < b->doms.size(); i++) {
+        b->doms[i]->batch_act = b->act + tiles;
         tiles += fill_batch_item(host.data() + ib * i, b->doms[i]->ka, b->doms[i]->tma, tiles, b->act);
+    }
     b->total_tiles = tiles;
     if (device_malloc(&b->items, host.size()) != cudaSuccess) {
         b->err = "cudaMalloc of the batch items failed";
