@@ -1948,13 +1948,18 @@ __global__ void __launch_bounds__(DTX *DTY, (Depth<Real, CPT>::MINB))
     __shared__ __align__(8) StencilShared<TS> sh;
     __shared__ __align__(16) KernelArgs sa;
     const int tid = threadIdx.y * DTX + threadIdx.x;
-    // the tile's domain: the domains that begin at or before it, less one
-    int d = -1;
-    for (int b = 0; b < nitems; b += 32) {
-        const int m = b + (int)threadIdx.x;
-        const unsigned in = __ballot_sync(FULL_MASK, m < nitems && items[m < nitems ? m : 0].tile_begin <= t);
-        d += __popc(in);
-        if (in != FULL_MASK) break;
+    // the tile's domain, the last that begins at or before it: a warp looks at
+    // 64 parts of what is left at once (one round of loads to 64 domains, two
+    // to 4096; 1200 domains of 16^3 in FP32: 516 us a step, 612 going through
+    // all of them 32 a round)
+    int d = 0;
+    for (int left = nitems; left > 1;) {
+        const int step = (left + 63) / 64, end = d + left;
+        const int m0 = d + (int)threadIdx.x * step, m1 = m0 + 32 * step;
+        const long long b0 = m0 < end ? items[m0].tile_begin : t + 1, b1 = m1 < end ? items[m1].tile_begin : t + 1;
+        const int part = (__popc(__ballot_sync(FULL_MASK, b0 <= t)) + __popc(__ballot_sync(FULL_MASK, b1 <= t)) - 1) * step;
+        d += part;
+        left = min(step, left - part);
     }
     const BatchItem &it = items[d];
     const int *src = (const int *)&it.a;
