@@ -424,7 +424,8 @@ int mms_batch_size(const mms_batch *b);
  * records (not for mms_step while it belongs to the batch). */
 mms_ctx *mms_batch_domain(mms_batch *b, int i);
 mms_status mms_batch_step(mms_batch *b, int nsteps);
-/* Stencil tile of that launch (as mms_set_stencil_tile). */
+/* Stencil tile of that launch (as mms_set_stencil_tile), and its grid: a CTA
+ * per tile of every domain. */
 mms_status mms_batch_set_stencil_tile(mms_batch *b, int cells_per_thread, int zchunk);
 mms_status mms_batch_get_stencil_tile(const mms_batch *b, int *cells_per_thread, int *zchunk, int *grid);
 /* Times the batched stencil for every tile candidate on shadows of the

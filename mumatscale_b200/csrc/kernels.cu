@@ -3282,23 +3282,17 @@ long long fill_batch_item(void *dst, const KernelArgs &a, const TmaHolder &tma, 
 }
 
 template <typename Real, int CPT>
-static int batch_grid_t()
+static void batch_prepare_t()
 {
     constexpr int bytes = Depth<Real, CPT>::TS * Stage<Real, CPT>::BYTES;
     cudaFuncSetAttribute(k_diffuse_fs_batch<Real, CPT, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     cudaFuncSetAttribute(k_diffuse_fs_batch<Real, CPT, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    int per_sm = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_diffuse_fs_batch<Real, CPT, true>, DTX * DTY, bytes);
-    int dev = 0, sms = 148;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    return (per_sm > 0 ? per_sm : 1) * sms;
 }
 
-int batch_grid(int precision, int cpt)
+void batch_prepare(int precision, int cpt)
 {
-    if (precision == MMS_PREC_F32) return cpt == 2 ? batch_grid_t<float, 2>() : batch_grid_t<float, 1>();
-    return cpt == 2 ? batch_grid_t<double, 2>() : batch_grid_t<double, 1>();
+    if (precision == MMS_PREC_F32) cpt == 2 ? batch_prepare_t<float, 2>() : batch_prepare_t<float, 1>();
+    else cpt == 2 ? batch_prepare_t<double, 2>() : batch_prepare_t<double, 1>();
 }
 
 // Blocks per domain of the batched small kernels (0 for a domain that

@@ -2503,7 +2503,7 @@ struct mms_batch {
     int *begin = nullptr;
     int totals[4] = {0, 0, 0, 0};
     int graph_totals[4] = {-1, -1, -1, -1};
-    int cpt = 1, zc = 0, grid = 0;
+    int cpt = 1, zc = 0;
     cudaGraphExec_t graph = nullptr;
     int graph_kernels = 0;
     uint64_t launches = 0;
@@ -2599,7 +2599,7 @@ mms_status batch_build_items(mms_batch *b)
     if (cudaMemcpyAsync(b->items, host.data(), host.size(), cudaMemcpyHostToDevice, b->stream) != cudaSuccess ||
         cudaStreamSynchronize(b->stream) != cudaSuccess)
         return MMS_ERR_CUDA;
-    b->grid = batch_grid(b->prec, b->cpt);
+    batch_prepare(b->prec, b->cpt);
     return batch_refresh(b);
 }
 
@@ -2822,7 +2822,7 @@ mms_status mms_batch_get_stencil_tile(const mms_batch *b, int *cells_per_thread,
     if (!b) return MMS_ERR_ARG;
     if (cells_per_thread) *cells_per_thread = b->cpt;
     if (zchunk) *zchunk = b->zc;
-    if (grid) *grid = b->grid;
+    if (grid) *grid = (int)std::min<long long>(b->total_tiles, 0x7fffffff);
     return MMS_OK;
 }
 
@@ -2908,7 +2908,7 @@ mms_status mms_batch_autotune(mms_batch *b, int reps, int *cells_per_thread, int
             if (!ok) continue;
             cudaMemcpyAsync(ditems, host.data(), host.size(), cudaMemcpyHostToDevice, b->stream);
             cudaStreamSynchronize(b->stream);
-            batch_grid(b->prec, cpt);  // the kernel's shared memory
+            batch_prepare(b->prec, cpt);
             std::vector<float> ms;
             for (int r = 0; r < reps + 2; r++) {
                 cudaEventRecord(e0, b->stream);

@@ -310,13 +310,13 @@ int launch_curv(const KernelArgs &a, int precision, void *stream);
 int launch_slab_phase(const KernelArgs &a, const TmaHolder &tma, int precision, void *stream, int phase,
                       int resume);
 // Batched stencil over many domains: one item per domain (opaque, built by
-// fill_batch_item, which returns the domain's tile count), one launch;
-// batch_grid: its CTAs resident at once.
+// fill_batch_item, which returns the domain's tile count), one launch of a
+// CTA per tile; batch_prepare: its shared memory, before the first launch.
 size_t batch_item_bytes();
 // (act: the batch's active-tile bytes, null: every tile)
 long long fill_batch_item(void *dst, const KernelArgs &a, const TmaHolder &tma, long long tile_begin,
                           unsigned char *act);
-int batch_grid(int precision, int cpt);
+void batch_prepare(int precision, int cpt);
 // act: the tiles to visit, a byte each over all domains (null: every tile)
 int launch_stencil_batch(const void *items, int nitems, long long total_tiles, int precision, int cpt,
                          const unsigned char *act, void *stream);

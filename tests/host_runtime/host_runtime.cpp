@@ -215,7 +215,6 @@ long long fill_batch_item(void *dst, const KernelArgs &a, const TmaHolder &, lon
     std::memcpy(dst, (const void *)&a.d, sizeof a.d);
     return a.d.tm.n;
 }
-int batch_grid(int, int) { return 148 * 3; }
 void batch_prepare(int, int) {}
 int launch_stencil_batch(const void *items, int n, long long, int, int, const unsigned char *act, void *)
 {

@@ -179,3 +179,16 @@ assert d.adjoint_gradient(target)["steps"] == 20
 d.close()
 assert stale() == 0 and held() == 0
 """)
+
+
+def test_the_grid_a_batch_reports(run):
+    """The CTAs of the stencil's launch: one per tile of every domain."""
+    run("""
+with M.Batch([p, p]) as b, M.Domain(p) as d:
+    for tile in ((1, 0), (2, 3), (1, 1)):
+        b.set_stencil_tile(*tile)
+        nx, ny, nz = p.grid
+        planes = tile[1] or 4  # (the stand-in's own choice)
+        tiles = -(-nx // (32 * tile[0])) * -(-ny // 8) * -(-nz // planes)
+        assert b.stencil_tile() == (*tile, 2 * tiles), (b.stencil_tile(), tiles)
+""")
