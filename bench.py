@@ -448,7 +448,7 @@ def ds256_workload(args) -> None:
         dom.set_profiling(False)
         out[form] = {"ms_total": ms, "launches": launches, "kernels": ks, "clocks": clk.summary(),
                      "tile": {"cells_per_thread": tile[0], "zchunk": tile[1], "cta_cells": [32 * tile[0], 8]},
-                     "visit_ms": tile[2], "grains": dom.num_grains, "timestep": dom.timestep}
+                     "grains": dom.num_grains, "timestep": dom.timestep, "all_tiles_ms": _all_tiles_ms(dom)}
         if form == "f64":
             # end to end through the public API with host buffers: upload the
             # whole state from pinned host memory, K steps each followed by a
@@ -495,10 +495,10 @@ def ds256_workload(args) -> None:
     value = ws * cells * K / (f64["ms_total"] / 1e3)
     value32 = ws * cells * K / (f32["ms_total"] / 1e3)
     peak, peak_kind = measured_peak_gbs()
-    # the stencil's HBM rate with every tile visited (the tuner's launches)
-    per_launch_s = f64["visit_ms"] / 1e3
-    achieved = BYTES_DIFFUSE["f64"] * cells / per_launch_s / 1e9
-    achieved32 = BYTES_DIFFUSE["f32"] * cells / (f32["visit_ms"] / 1e3) / 1e9
+    # the stencil's HBM rate with every tile visited
+    achieved = BYTES_DIFFUSE["f64"] * cells / (f64["all_tiles_ms"] / 1e3) / 1e9
+    achieved32 = BYTES_DIFFUSE["f32"] * cells / (f32["all_tiles_ms"] / 1e3) / 1e9
+    st_ms, st_n = f64["kernels"]["k_diffuse_fs"]
     tr = ncu_traffic_per_cell("f64")
     step_ms = f64["ms_total"] / K
     share = {k: round(v[0] / max(1e-9, sum(x[0] for x in f64["kernels"].values())), 4)
@@ -528,7 +528,8 @@ def ds256_workload(args) -> None:
                      "unit": "GB/s", "frac": achieved / peak, "peak_source": peak_kind,
                      "algorithmic_bytes_per_cell": BYTES_DIFFUSE["f64"],
                      "traffic": (tr * cells) if tr else None,
-                     "kernel_ms_per_launch": per_launch_s * 1e3},
+                     "kernel_ms_per_launch": st_ms / max(st_n, 1),
+                     "all_tiles_ms_per_launch": f64["all_tiles_ms"]},
         "kernel_share": share,
         "e2e": out["e2e"],
         "gpu_launches": f64["launches"],
@@ -585,16 +586,29 @@ def _dist(ws):
     return barrier, max_over_ranks
 
 
-def _roofline(ks: dict, steps: int, cells: int, form: str, peaks: dict, visit_ms: float) -> dict:
+def _all_tiles_ms(dom, reps: int = 5) -> float:
+    """Device time of the steps' own stencil kernel in a step that visits every
+    tile, which is the step after an upload (of the grain ids as they stand):
+    median of `reps` steps."""
+    ms = []
+    for _ in range(reps):
+        dom.upload("gr", dom.download("gr"))
+        dom.set_profiling(True)
+        dom.step(1)
+        total, n = dom.kernel_stats()["k_diffuse_fs"]
+        dom.set_profiling(False)
+        ms.append(total / n)
+    return sorted(ms)[reps // 2]
+
+
+def _roofline(ks: dict, steps: int, cells: int, form: str, peaks: dict, all_tiles_ms: float) -> dict:
     """Roofline of the kernel with the largest device time in ks
     (name -> (ms over `steps` steps, launches)).  The stencil leaves tiles at
-    rest out, so its HBM rate is that of a launch that visits every tile
-    (visit_ms, the tuner's time of the chosen tile)."""
+    rest out, so its HBM rate is that of its launches that visit every tile
+    (all_tiles_ms); kernel_ms_per_launch is the run's own."""
     name = max(ks, key=lambda k: ks[k][0])
     ms, n = ks[name]
     per_launch = ms / 1e3 / max(n, 1)
-    if name == "k_diffuse_fs":
-        per_launch = visit_ms / 1e3
     if name == "k_temp_am":
         # tables + contraction per step: 2 x 400 multiply-adds per cell the
         # step computes (x = 1..gx of every halo'd (y, z) row; the halo
@@ -611,13 +625,15 @@ def _roofline(ks: dict, steps: int, cells: int, form: str, peaks: dict, visit_ms
                 "peak_source": peaks["source"] + " (dense bf16 GEMM)",
                 "algorithmic_flops_per_launch": flops, "traffic": None,
                 "kernel_ms_per_launch": per_launch * 1e3}
-    b = BYTES_DIFFUSE_AM[form] if name == "k_diffuse_fs" else BYTES_STEP[form]
-    ach = b * cells / per_launch / 1e9
+    stencil = name == "k_diffuse_fs"
+    b = BYTES_DIFFUSE_AM[form] if stencil else BYTES_STEP[form]
+    ach = b * cells / (all_tiles_ms / 1e3 if stencil else per_launch) / 1e9
     tr = ncu_traffic_per_cell(form, "am")
     return {"bound": "hbm", "kernel": name, "achieved": ach, "peak": peaks["hbm_gbs"], "unit": "GB/s",
             "frac": ach / peaks["hbm_gbs"], "peak_source": peaks["source"],
             "algorithmic_bytes_per_cell": b, "traffic": (tr * cells) if tr else None,
-            "kernel_ms_per_launch": per_launch * 1e3}
+            "kernel_ms_per_launch": per_launch * 1e3,
+            "all_tiles_ms_per_launch": all_tiles_ms if stencil else None}
 
 
 def gpu_arm(args) -> None:
@@ -661,7 +677,7 @@ def gpu_arm(args) -> None:
         ms = max_over_ranks(e0.elapsed_time(e1))
         out[form] = {"ms_total": ms, "launches": dom.kernel_launches - l0, "clocks": clk.summary(),
                      "tile": {"cells_per_thread": tile[0], "zchunk": tile[1], "cta_cells": [32 * tile[0], 8]},
-                     "visit_ms": tile[2], "grains": dom.num_grains - 1}
+                     "grains": dom.num_grains - 1}
         if form == "f32":
             out[form]["tile"]["am_rows"] = dom.am_tile()
         doms[form] = dom
@@ -673,6 +689,7 @@ def gpu_arm(args) -> None:
         torch.cuda.synchronize()
         out[form]["kernels"] = dom.kernel_stats()
         dom.set_profiling(False)
+        out[form]["all_tiles_ms"] = _all_tiles_ms(dom)
         dom.close()
     del doms
 
@@ -721,10 +738,10 @@ def gpu_arm(args) -> None:
     value64 = ws * cells * K / (f64["ms_total"] / 1e3)
     peak, peak_kind = measured_peak_gbs()
     peaks = {"hbm_gbs": peak, "bf16_tflops": measured_peak_tflops(), "source": peak_kind}
-    roof = _roofline(f32["kernels"], K, cells, "f32", peaks, f32["visit_ms"])
-    # the stencil's HBM rate with every tile visited (the tuner's launches)
-    st32 = BYTES_DIFFUSE_AM["f32"] * cells / (f32["visit_ms"] / 1e3) / 1e9
-    st64 = BYTES_DIFFUSE_AM["f64"] * cells / (f64["visit_ms"] / 1e3) / 1e9
+    roof = _roofline(f32["kernels"], K, cells, "f32", peaks, f32["all_tiles_ms"])
+    # the stencil's HBM rate with every tile visited
+    st32 = BYTES_DIFFUSE_AM["f32"] * cells / (f32["all_tiles_ms"] / 1e3) / 1e9
+    st64 = BYTES_DIFFUSE_AM["f64"] * cells / (f64["all_tiles_ms"] / 1e3) / 1e9
 
     def per_step(ks):
         return {k: round(v[0] / K, 5) for k, v in ks.items() if v[1]}
@@ -796,7 +813,7 @@ def ds256_device(args, ws, stream, barrier, max_over_ranks) -> dict:
     for form, prec in (("f64", M.PREC_F64), ("f32", M.PREC_F32)):
         with M.Domain(params, precision=prec) as dom:
             dom.set_stream(stream.cuda_stream)
-            visit_ms = dom.autotune(reps=3)[2]
+            dom.autotune(reps=3)
             dom.step(Wm)
             torch.cuda.synchronize()
             barrier()
@@ -806,8 +823,8 @@ def ds256_device(args, ws, stream, barrier, max_over_ranks) -> dict:
             e1.record(stream)
             torch.cuda.synchronize()
             ms = max_over_ranks(e0.elapsed_time(e1))
-            # the stencil's HBM rate with every tile visited (the tuner's launches)
-            gbs = BYTES_DIFFUSE[form] * N_CELL ** 3 / (visit_ms / 1e3) / 1e9
+            # the stencil's HBM rate with every tile visited
+            gbs = BYTES_DIFFUSE[form] * N_CELL ** 3 / (_all_tiles_ms(dom) / 1e3) / 1e9
             out[form] = {"value": ws * N_CELL ** 3 * K / (ms / 1e3), "ms_per_step": ms / K,
                          "k_diffuse_fs_gbs": gbs, "k_diffuse_fs_frac": gbs / measured_peak_gbs()[0]}
     out["workload"] = "multi-grain directional solidification, 256^3 cells"
@@ -998,7 +1015,7 @@ def ensemble_workload(args) -> None:
                 "metric": UNIT, "unit": UNIT, "value": cells_all * steps / sec, "n_gpus": ws, "steps": steps,
                 "warmup": args.warmup, "cells_total": cells_all, "ms_per_step": sec * 1e3 / steps,
                 "scaling": "strong", "data": "synthetic",
-                "tile": {"cells_per_thread": tile[0], "zchunk": tile[1], "persistent_ctas": tile[2],
+                "tile": {"cells_per_thread": tile[0], "zchunk": tile[1], "ctas": tile[2],
                          "tuned_stencil_ms": tune[2]},
                 "grains_rank0": grains, "kernel_launches_per_step": launches / max(1, steps + args.warmup),
                 "sequential_domains": seq,
