@@ -448,7 +448,7 @@ def ds256_workload(args) -> None:
         dom.set_profiling(False)
         out[form] = {"ms_total": ms, "launches": launches, "kernels": ks, "clocks": clk.summary(),
                      "tile": {"cells_per_thread": tile[0], "zchunk": tile[1], "cta_cells": [32 * tile[0], 8]},
-                     "grains": dom.num_grains, "timestep": dom.timestep, "all_tiles_ms": _all_tiles_ms(dom)}
+                     "grains": dom.num_grains, "timestep": dom.timestep, "visits": _stencil_visits(dom, K)}
         if form == "f64":
             # end to end through the public API with host buffers: upload the
             # whole state from pinned host memory, K steps each followed by a
@@ -495,9 +495,8 @@ def ds256_workload(args) -> None:
     value = ws * cells * K / (f64["ms_total"] / 1e3)
     value32 = ws * cells * K / (f32["ms_total"] / 1e3)
     peak, peak_kind = measured_peak_gbs()
-    # the stencil's HBM rate with every tile visited
-    achieved = BYTES_DIFFUSE["f64"] * cells / (f64["all_tiles_ms"] / 1e3) / 1e9
-    achieved32 = BYTES_DIFFUSE["f32"] * cells / (f32["all_tiles_ms"] / 1e3) / 1e9
+    achieved = _stencil_gbs(f64["visits"], BYTES_DIFFUSE["f64"], cells)
+    achieved32 = _stencil_gbs(f32["visits"], BYTES_DIFFUSE["f32"], cells)
     st_ms, st_n = f64["kernels"]["k_diffuse_fs"]
     tr = ncu_traffic_per_cell("f64")
     step_ms = f64["ms_total"] / K
@@ -527,9 +526,9 @@ def ds256_workload(args) -> None:
         "roofline": {"bound": "hbm", "kernel": "k_diffuse_fs", "achieved": achieved, "peak": peak,
                      "unit": "GB/s", "frac": achieved / peak, "peak_source": peak_kind,
                      "algorithmic_bytes_per_cell": BYTES_DIFFUSE["f64"],
-                     "traffic": (tr * cells) if tr else None,
+                     "traffic": (tr * cells * f64["visits"][1]) if tr else None,
                      "kernel_ms_per_launch": st_ms / max(st_n, 1),
-                     "all_tiles_ms_per_launch": f64["all_tiles_ms"]},
+                     "visited_fraction": f64["visits"][1]},
         "kernel_share": share,
         "e2e": out["e2e"],
         "gpu_launches": f64["launches"],
@@ -586,26 +585,31 @@ def _dist(ws):
     return barrier, max_over_ranks
 
 
-def _all_tiles_ms(dom, reps: int = 5) -> float:
-    """Device time of the steps' own stencil kernel in a step that visits every
-    tile, which is the step after an upload (of the grain ids as they stand):
-    median of `reps` steps."""
-    ms = []
-    for _ in range(reps):
-        dom.upload("gr", dom.download("gr"))
+def _stencil_visits(dom, steps: int) -> tuple[float, float]:
+    """(ms per launch of the steps' stencil kernel, mean fraction of the
+    domain's tiles that it visited) over `steps` steps, profiled one by one."""
+    ms = share = 0.0
+    for _ in range(steps):
         dom.set_profiling(True)
         dom.step(1)
         total, n = dom.kernel_stats()["k_diffuse_fs"]
         dom.set_profiling(False)
-        ms.append(total / n)
-    return sorted(ms)[reps // 2]
+        tiles, left_out = dom.test_tile_map()
+        ms += total / n
+        share += 1.0 - left_out / tiles if tiles else 1.0
+    return ms / steps, share / steps
 
 
-def _roofline(ks: dict, steps: int, cells: int, form: str, peaks: dict, all_tiles_ms: float) -> dict:
+def _stencil_gbs(visits: tuple[float, float], bytes_per_cell: float, cells: int) -> float:
+    """The stencil's HBM rate: the fields' bytes in the tiles it visited."""
+    return bytes_per_cell * cells * visits[1] / (visits[0] / 1e3) / 1e9
+
+
+def _roofline(ks: dict, steps: int, cells: int, form: str, peaks: dict, visits: tuple[float, float]) -> dict:
     """Roofline of the kernel with the largest device time in ks
     (name -> (ms over `steps` steps, launches)).  The stencil leaves tiles at
-    rest out, so its HBM rate is that of its launches that visit every tile
-    (all_tiles_ms); kernel_ms_per_launch is the run's own."""
+    rest out: its rate counts the tiles it visited (visits, of the same
+    run's steps: _stencil_visits)."""
     name = max(ks, key=lambda k: ks[k][0])
     ms, n = ks[name]
     per_launch = ms / 1e3 / max(n, 1)
@@ -627,13 +631,13 @@ def _roofline(ks: dict, steps: int, cells: int, form: str, peaks: dict, all_tile
                 "kernel_ms_per_launch": per_launch * 1e3}
     stencil = name == "k_diffuse_fs"
     b = BYTES_DIFFUSE_AM[form] if stencil else BYTES_STEP[form]
-    ach = b * cells / (all_tiles_ms / 1e3 if stencil else per_launch) / 1e9
+    ach = _stencil_gbs(visits, b, cells) if stencil else b * cells / per_launch / 1e9
     tr = ncu_traffic_per_cell(form, "am")
     return {"bound": "hbm", "kernel": name, "achieved": ach, "peak": peaks["hbm_gbs"], "unit": "GB/s",
             "frac": ach / peaks["hbm_gbs"], "peak_source": peaks["source"],
-            "algorithmic_bytes_per_cell": b, "traffic": (tr * cells) if tr else None,
+            "algorithmic_bytes_per_cell": b, "traffic": (tr * cells * (visits[1] if stencil else 1.0)) if tr else None,
             "kernel_ms_per_launch": per_launch * 1e3,
-            "all_tiles_ms_per_launch": all_tiles_ms if stencil else None}
+            "visited_fraction": visits[1] if stencil else None}
 
 
 def gpu_arm(args) -> None:
@@ -689,7 +693,7 @@ def gpu_arm(args) -> None:
         torch.cuda.synchronize()
         out[form]["kernels"] = dom.kernel_stats()
         dom.set_profiling(False)
-        out[form]["all_tiles_ms"] = _all_tiles_ms(dom)
+        out[form]["visits"] = _stencil_visits(dom, K)
         dom.close()
     del doms
 
@@ -738,10 +742,9 @@ def gpu_arm(args) -> None:
     value64 = ws * cells * K / (f64["ms_total"] / 1e3)
     peak, peak_kind = measured_peak_gbs()
     peaks = {"hbm_gbs": peak, "bf16_tflops": measured_peak_tflops(), "source": peak_kind}
-    roof = _roofline(f32["kernels"], K, cells, "f32", peaks, f32["all_tiles_ms"])
-    # the stencil's HBM rate with every tile visited
-    st32 = BYTES_DIFFUSE_AM["f32"] * cells / (f32["all_tiles_ms"] / 1e3) / 1e9
-    st64 = BYTES_DIFFUSE_AM["f64"] * cells / (f64["all_tiles_ms"] / 1e3) / 1e9
+    roof = _roofline(f32["kernels"], K, cells, "f32", peaks, f32["visits"])
+    st32 = _stencil_gbs(f32["visits"], BYTES_DIFFUSE_AM["f32"], cells)
+    st64 = _stencil_gbs(f64["visits"], BYTES_DIFFUSE_AM["f64"], cells)
 
     def per_step(ks):
         return {k: round(v[0] / K, 5) for k, v in ks.items() if v[1]}
@@ -770,9 +773,11 @@ def gpu_arm(args) -> None:
         "parallelism": f"replicas x{ws}",
         "fp64_plain": {"value": value64, "ms_per_step": f64["ms_total"] / K, "grains_after_run": f64["grains"],
                        "k_diffuse_fs_gbs": st64, "k_diffuse_fs_frac": st64 / peak,
+                       "visited_fraction": f64["visits"][1],
                        "kernel_ms_per_step": per_step(f64["kernels"]), "stencil_tile": f64["tile"]},
         "fp32_form": {"ratio_vs_fp64": value / value64, "errors_vs_fp64": errors,
                       "k_diffuse_fs_gbs": st32, "k_diffuse_fs_frac": st32 / peak,
+                      "visited_fraction": f32["visits"][1],
                       "kernel_ms_per_step": per_step(f32["kernels"]), "stencil_tile": f32["tile"]},
         "roofline": roof,
         "e2e": e2e,
@@ -823,8 +828,7 @@ def ds256_device(args, ws, stream, barrier, max_over_ranks) -> dict:
             e1.record(stream)
             torch.cuda.synchronize()
             ms = max_over_ranks(e0.elapsed_time(e1))
-            # the stencil's HBM rate with every tile visited
-            gbs = BYTES_DIFFUSE[form] * N_CELL ** 3 / (_all_tiles_ms(dom) / 1e3) / 1e9
+            gbs = _stencil_gbs(_stencil_visits(dom, K), BYTES_DIFFUSE[form], N_CELL ** 3)
             out[form] = {"value": ws * N_CELL ** 3 * K / (ms / 1e3), "ms_per_step": ms / K,
                          "k_diffuse_fs_gbs": gbs, "k_diffuse_fs_frac": gbs / measured_peak_gbs()[0]}
     out["workload"] = "multi-grain directional solidification, 256^3 cells"
