@@ -147,8 +147,9 @@ __device__ __forceinline__ void fence_barrier_init()
 // Z_i(z) = ldt exp(-lz^2/b_i) / Tl_i, built once per step (k_am_tables),
 // instead of 400 exponentials per cell (k_am_contract).  Cells above the
 // substrate top (rz > znow + dx) get T = 0.
+
 // Largest X, Y and Z of every node over each column, row and layer of stencil
-// tiles, for the tiles' temperature bound (tile_keeps): the Gaussian at the
+// tiles, for the tiles' temperature bound (tile_scan): the Gaussian at the
 // point of the interval nearest its centre.
 __device__ __forceinline__ void am_tile_max(const KernelArgs &a, const AmParams &m, const AmStep &s, unsigned first,
                                             unsigned stride)
@@ -430,8 +431,8 @@ __global__ void __launch_bounds__(AMC_NT, 2) k_am_contract(KernelArgs a, AmParam
 // x 128 FP32 118 -> 86 us.  With every tile active the difference is within
 // the runs' spread.
 
-// T over a tile's planes, analytic models that depend on z alone: the value is
-// monotone in z, as rounded, so its extremes are those of the end planes.
+// Whether kept-solid cells (fs_update) keep their branch at every T in [lo, hi],
+// x the least of their m (cl - Cinit): the tests and roundings of fs_update.
 template <typename Real>
 __device__ __forceinline__ bool keeps_at(const Phys &p, double lo, double hi, double x)
 {
@@ -500,6 +501,8 @@ __device__ __forceinline__ void tile_scan(const KernelArgs &a, int blk)
             const double hi = head[0] + head[1] * (1.001 * (double)sum) + 0.01;
             keeps = head[1] >= 0.0 && keeps_at<Real>(p, head[0] - 0.01, hi, x);
         } else if (p.temp_mode == 0 || !p.gz_is_one) {
+            // T depends on z alone and is monotone in it, as rounded: its
+            // extremes are those of the end planes
             const int k0 = bz * tm.zc + 1, k1 = min(k0 + tm.zc - 1, g.gz);
             const double T0 = temp_cell(p, nullptr, nullptr, 0, 1, k0, ts);
             const double T1 = temp_cell(p, nullptr, nullptr, 0, 1, k1, ts);
@@ -1314,9 +1317,8 @@ struct TmaMaps {
     CUtensorMap cl[2], fs[2], ce, gr;
 };
 
-// Shared-memory state of a stencil CTA, kept across the tiles a persistent
-// CTA processes: the ring, one mbarrier per slot (initialised once), the
-// per-plane temperatures and the abort flag.
+// Shared-memory state of a stencil CTA: one mbarrier per ring slot, the
+// per-plane temperatures, the warps' sums and the abort flag.
 template <int TS>
 struct StencilShared {
     unsigned long long bars[TS];
@@ -2510,17 +2512,22 @@ __device__ __forceinline__ void capture_body(const KernelArgs &a, int bid, int n
     }
 }
 
-// The same with eight lanes per entry, for domains whose lists are so short
-// that every entry is in flight at once either way: a thread per entry goes
-// through the loads of a neighbour's rotation, octahedron centre and fs once
-// for each solid neighbour.  Lanes 0-5 test one neighbour each, in the reference's order (+x,
-// +y, -x, -y, +z, -z; growth.c:604-610, 674-677), and the first that reaches
-// the cell commits; lane 6 has fetched the entry's dc_tmp slot meanwhile and
-// commits that when none does.  64^3 one-grain deck, 700 entries, event timing:
-// 16.1 -> 10.6 us; with 166,000 entries (melt pool 512 x 256 x 128) the
-// eightfold instructions tell, 20 against 56 us, and at 58,000 the two are
-// equal, so only domains of at most 2^18 cells take it, whose lists stay below
-// that until almost a quarter of the cells is interface.
+// The same with eight lanes per entry, for small domains: a thread per entry
+// goes through the loads of a neighbour's rotation, octahedron centre and fs
+// once for each solid neighbour.  Lanes 0-5 test one neighbour each, in the
+// reference's order (+x, +y, -x, -y, +z, -z; growth.c:604-610, 674-677), and the
+// first that reaches the cell commits; lane 6 has fetched the entry's dc_tmp
+// slot meanwhile and commits that when none does.
+// Event timing, a thread -> eight lanes per entry: 64^3 with one grain, 700
+// entries, 16.1 -> 10.6 us; with 20,000 grains, 134,000 entries of 1.9 solid
+// neighbours each 31.4 -> 26.2 us, 72,000 of 3.1 26.2 -> 18.9.  It loses on long
+// lists around grains of one cell, whose entries have one solid neighbour each
+// and go through one round of loads either way: 87,000 of 1.2 16.9 -> 19.7, which
+// is the first few dozen steps of such a run; a thread per entry beyond a list
+// length instead gave up more in the later states than it saved there.  At
+// 166,000 entries over a flat substrate (melt pool 512 x 256 x 128) 20 -> 56, so
+// only domains of at most 2^18 cells take it.  (Four, six and eight blocks an SM:
+// 15 to 30 % slower on long lists.)
 constexpr int CAP_LANES = 8;
 constexpr long long CAP_LANES_CELLS = 1LL << 18;  // largest domain that takes it
 template <typename Real>
