@@ -2939,8 +2939,9 @@ static int pick_zchunk(const Geo &g, int tile_x)
     // (64-wide tiles: at most 8, which leaves more of them to run at once and
     // finer ones to leave out; us per step, 8 / 16 / 32 planes: 256^3 FP64
     // 218 / 223 / 244, FP32 139 / 140 / 149, 512 x 256 x 128 melt pool FP32
-    // 257 / 268 / 267)
-    if (zc > (tile_x > DTX ? 8 : 32)) zc = tile_x > DTX ? 8 : 32;
+    // 257 / 268 / 267; more where a grid would have over 65,535 layers of tiles)
+    const int most = std::max(tile_x > DTX ? 8 : 32, (g.gz + 65534) / 65535);
+    if (zc > most) zc = most;
     if (zc > g.gz) zc = g.gz;
     return zc;
 }
