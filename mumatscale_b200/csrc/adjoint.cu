@@ -414,12 +414,14 @@ static int adj_blocks(const Geo &g) { return (int)(((long long)g.gx * g.gy * g.g
 // above and below, short ones give a small domain enough CTAs.  A gradient over
 // 100 steps of 128^3 in FP64: 13.9, 11.6, 10.6, 10.8 and 10.7 ms with 1, 2, 4, 6
 // and 11 planes (16: a fifth slower); over 40 steps of 57 x 63 x 49 in FP32:
-// 0.79, 0.76, 0.89, 1.00 and 1.41 ms.
+// 0.79, 0.76, 0.89, 1.00 and 1.41 ms.  More where a grid would have over 65,535
+// layers of them.
 static int adj_zc(const Geo &g)
 {
     const long long tiles = (long long)((g.gx + ADX - 1) / ADX) * ((g.gy + ADY - 1) / ADY);
     const long long zc = tiles * g.gz / (148 * 3);
-    return (int)(zc < 1 ? 1 : (zc > 6 ? 6 : zc));
+    const int least = (g.gz + 65534) / 65535;
+    return std::max(least, (int)(zc < 1 ? 1 : (zc > 6 ? 6 : zc)));
 }
 
 static dim3 adj_grid(const Geo &g, int zc)

@@ -34,3 +34,18 @@ def test_default_tile_of_a_tall_domain(built, cuda_device, tmp_path):
         dom.set_stencil_tile(1, 32)
         dom.step(3)
         assert np.array_equal(gr, dom.download("gr")) and np.array_equal(ce, dom.download("ce"))
+
+
+def test_adjoint_of_a_tall_domain(built, cuda_device, tmp_path):
+    dims = (3, 3, 65535 * 6 + 50)
+    with _domain(tmp_path, dims, M.PREC_F64) as dom:
+        target = dom.download("ce")
+        dom.step(2)
+        dom.adjoint_record(4, 2)
+        assert dom.adjoint_replay_loss(dom.download("ce")) == 0.0
+        g = dom.adjoint_gradient(target)
+        assert g["loss"] > 0 and g["Dliq"] != 0
+        assert abs(g["loss"] - dom.adjoint_replay_loss(target)) <= 1e-13 * g["loss"]
+        up, dn = (dom.adjoint_replay_loss(target, (1 + s, 1.0, 1.0)) for s in (1e-4, -1e-4))
+        fd = (up - dn) / 2e-4
+        assert abs(g["Dliq"] * dom.params.Dliq - fd) <= 1e-4 * abs(fd)  # as in test_adjoint
