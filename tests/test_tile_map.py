@@ -177,3 +177,43 @@ def test_map_with_resumed_steps(built, cuda_device, tmp_path, monkeypatch, prec)
             assert dom.test_tile_map()[0] == _tiles(1, 5)
             _same(dom, every, n)
         assert dom.num_grains == every.num_grains > 600
+
+
+@pytest.mark.parametrize("prec", [M.PREC_F64, M.PREC_F32])
+def test_map_without_sites(built, cuda_device, tmp_path, monkeypatch, prec):
+    """A microstructure that only grows and melts."""
+    p = _params(tmp_path, monkeypatch, "heating")
+    planes = T.KINDS["heating"][3]
+    rot = np.stack([W.quat_to_rotmat(q).ravel() for q in W.random_quaternions(np.random.default_rng(1), 1)])
+    gr = np.zeros(tuple(n + 2 for n in DIMS[::-1]), dtype=np.int32)
+    gr[1:planes + 1, 1:-1, 1:-1] = 1
+    with M.Domain(p, precision=prec) as dom, M.SlabGroup(p, 2, precision=prec) as every:
+        dom.set_stencil_tile(2, 3)
+        for d in (dom, every):
+            d.set_grains(rot)
+            d.upload("gr", gr)
+            d.upload("fs", (gr > 0).astype(np.float64))
+        counts = []
+        for n in (1, 60, 90, 60):
+            dom.step(n)
+            every.step(n)
+            counts.append(dom.test_tile_map()[1])
+            _same(dom, every, n)
+        _left_out(counts, "heating")
+
+
+@pytest.mark.parametrize("kind", ["cooling", "heating", "laser"])
+@pytest.mark.parametrize("prec", [M.PREC_F64, M.PREC_F32])
+def test_slabs_with_wide_default_tiles(built, cuda_device, tmp_path, monkeypatch, kind, prec):
+    """Slabs large enough for two cells per thread by default, against one
+    domain with one."""
+    dims = (250, 128, 126)
+    p = _params(tmp_path, monkeypatch, kind, dims)
+    with M.Domain(p, precision=prec) as dom, M.SlabGroup(p, 2, precision=prec) as every:
+        dom.set_stencil_tile(1, 16)
+        assert every.slabs[0].stencil_tile() == (2, 0)
+        _setup((dom, every), kind, dims)
+        for n in (1, 2, 67, 70):
+            dom.step(n)
+            every.step(n)
+            _same(dom, every, n)
