@@ -11,6 +11,8 @@ cells); with k = 0.14 every deck here uses D_l dt / dx^2 = 0.04.
 """
 from __future__ import annotations
 
+import math
+
 import numpy as np
 
 T_MELT = 933.47
@@ -21,9 +23,23 @@ T_SOL = T_MELT + SLOPE * C0 / K_PART
 FOURIER = 0.04  # D_l dt / dx^2
 
 
+def _norm(q) -> float:
+    """Euclidean norm, each square added with one rounding (a fused multiply-add).
+    numpy's BLAS does so on some hosts and rounds the squares first on others,
+    where the rotations of the same seed would differ in their last bits."""
+    s = 0.0
+    for v in map(float, q):
+        hi = v * 134217729.0  # Veltkamp's split at 27 bits, Dekker's exact product
+        hi -= hi - v
+        lo = v - hi
+        p = v * v
+        s = math.fsum((p, ((hi * hi - p) + 2.0 * hi * lo) + lo * lo, s))
+    return math.sqrt(s)
+
+
 def quat_to_rotmat(q) -> np.ndarray:
     """Row-major 3x3 rotation matrix of a (w, x, y, z) quaternion (normalised here)."""
-    w, x, y, z = np.asarray(q, dtype=np.float64) / np.linalg.norm(q)
+    w, x, y, z = np.asarray(q, dtype=np.float64) / _norm(q)
     return np.array([[1 - 2 * (y * y + z * z), 2 * (x * y - z * w), 2 * (x * z + y * w)],
                      [2 * (x * y + z * w), 1 - 2 * (x * x + z * z), 2 * (y * z - x * w)],
                      [2 * (x * z - y * w), 2 * (y * z + x * w), 1 - 2 * (x * x + y * y)]])
