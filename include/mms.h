@@ -400,7 +400,8 @@ mms_status mms_get_stencil_tile(const mms_ctx *ctx, int *cells_per_thread, int *
 mms_status mms_set_am_tile(mms_ctx *ctx, int rows);
 mms_status mms_get_am_tile(const mms_ctx *ctx, int *rows);
 /* Times every tile candidate on shadow copies of the fields the stencil
- * writes (the domain's state is left as it was), keeps the fastest by median
+ * writes (the domain's state is left as it was), each launch visiting the whole
+ * domain, where a step leaves tiles at rest out; keeps the fastest by median
  * of `reps` launches and returns it (any output pointer may be NULL).  For
  * the FP32 form of the moving-source (AM) temperature model it also picks
  * the tensor-core contraction's tile (128 x cells by 128 or 256 rows or the default), timed
